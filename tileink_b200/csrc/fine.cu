@@ -1,4 +1,5 @@
-// Fine stage: one CTA of 256 threads per 16x16 tile, one thread per pixel
+// Fine stage of scenes with SDF records or text (the others take
+// fine_paths.cu): one CTA of 256 threads per 16x16 tile, one thread per pixel
 // (fine/main.hlsl:23-40, fine/interpreter.hlsli:21-219,
 // fine/specialized.hlsli:19-45).
 //
@@ -24,6 +25,7 @@
 #include <cuda_runtime.h>
 
 #include "device.cuh"
+#include "fine.cuh"
 #include "kernels.h"
 #include "sdf.cuh"
 #include "text.cuh"
@@ -38,16 +40,6 @@ constexpr uint32_t kRecChunk = 64;
 constexpr uint32_t kSegBudget = 128;
 constexpr uint32_t kProdCap = 2560;
 static_assert(kRecChunk <= 64u && kSegBudget <= 256u, "offsets are scanned by one warp, two records a lane");
-constexpr uint32_t kClipSpill = 28;
-constexpr uint32_t kGroupDepth = 6;
-constexpr uint32_t kGroupLocal = 2;  // FINE_LOCAL_GROUP_DEPTH (fine/constants.hlsli:11)
-constexpr uint32_t kGradient = 0xFFFFFFFFu;
-constexpr uint32_t kGradParams = 24;
-constexpr uint32_t kGradConst = 0, kGradLinear = 1, kGradRadial = 2, kGradPattern = 3;  // decoded kinds
-constexpr uint32_t kGradBilinear = 1u << 16;  // pattern: bilinear sampling
-constexpr uint32_t kGradDenOk = 1u << 16;    // linear: den > GRADIENT_FLOAT_EPSILON
-constexpr uint32_t kGradASmall = 1u << 16;   // radial: |a| <= RADIAL_QUADRATIC_EPSILON
-
 // Record classes driving the per-pixel dispatch.
 constexpr uint32_t kClsOther = 0, kClsFill = 1, kClsUniform = 2, kClsBatch = 3, kClsEnd = 4;
 
@@ -88,11 +80,6 @@ struct FineSmem {
     uint32_t n, nprod;
 };
 
-__device__ __forceinline__ bool is_fill_like(uint32_t tag) {
-    return tag == TK_PTCL_FILL || tag == TK_PTCL_BEGIN_CLIP || tag == TK_PTCL_BEGIN_OPACITY ||
-           tag == TK_PTCL_BEGIN_BLEND || tag == TK_PTCL_PATH_GLYPH;
-}
-
 __device__ __forceinline__ float4 texel_load_lut(const FineSmem& S, uint32_t p) {
     return make_float4(S.unorm[p & 255u], S.unorm[(p >> 8) & 255u], S.unorm[(p >> 16) & 255u], S.unorm[p >> 24]);
 }
@@ -102,8 +89,8 @@ __device__ __forceinline__ float4 texel_load_lut(const FineSmem& S, uint32_t p) 
 // sample_gradient (fine/paint.hlsli:40-96) that depend on the brush alone,
 // computed with the same f32 operations so that the per-pixel evaluation in
 // gradient_at gives the same bits.
-//   linear: gp[12..16] = sx, sy, dx = ex - sx, dy = ey - sy, den = dx*dx + dy*dy
-//   radial: gp[12..22] = sx, sy, dcx, dcy, sr*dr, -sr*sr, a, -4*a, 2*a, dr, sr
+//   linear: gp[12..17] = sx, sy, dx = ex - sx, dy = ey - sy, den = dx*dx + dy*dy, 1/den
+//   radial: gp[12..23] = sx, sy, dcx, dcy, sr*dr, -sr*sr, a, -4*a, 2*a, dr, sr, 1/(2*a)
 //           with a = mad(dcx, dcx, mad(dcy, dcy, -dr*dr))
 __device__ void decode_gradient(float* g, uint4& gk, const Paint& P, uint32_t db, const float* __restrict__ m,
                                 const uint4* __restrict__ images, uint32_t image_count) {
@@ -126,6 +113,8 @@ __device__ void decode_gradient(float* g, uint4& gk, const Paint& P, uint32_t db
         g[15] = dy;
         g[16] = den;
         if (den > GRADIENT_FLOAT_EPSILON) flags = kGradDenOk;
+        g[17] = 1.0f / den;
+        if (divisor_is_plain(den)) flags |= kGradFast;
         word = payload;
     } else if (kind == TK_BRUSH_RADIAL) {
         code = kGradRadial;
@@ -146,6 +135,8 @@ __device__ void decode_gradient(float* g, uint4& gk, const Paint& P, uint32_t db
         g[21] = dr;
         g[22] = sr;
         if (fabsf(a) <= RADIAL_QUADRATIC_EPSILON) flags = kGradASmall;
+        g[23] = 1.0f / g[20];
+        if (divisor_is_plain(g[20])) flags |= kGradFast;
         word = payload;
     } else if (kind == TK_BRUSH_PATTERN_RESOURCE) {
         // sample_brush's texture-table branch (shared/brush/sample.hlsli:32-41):
@@ -167,6 +158,14 @@ __device__ void decode_gradient(float* g, uint4& gk, const Paint& P, uint32_t db
     } else {
         word = kind == 6u ? 0u : P.word(db + TK_BRUSH_COLOR_WORD);  // BRUSH_PATTERN samples as 0
     }
+    if ((code == kGradLinear || code == kGradRadial) && len > 1u && len < (1u << 22) &&
+        uint64_t(word) + len <= P.count)
+        flags |= kGradRampOk;
+    bool identity = code == kGradLinear || code == kGradRadial;
+    for (int t = 0; t < 12; t += 6)
+        identity = identity && g[t] == 1.0f && g[t + 1] == 0.0f && g[t + 2] == 0.0f && g[t + 3] == 1.0f &&
+                   g[t + 4] == 0.0f && g[t + 5] == 0.0f;
+    if (identity) flags |= kGradIdentity;
     gk = make_uint4(code | flags, word, len, extend);
 }
 
@@ -192,126 +191,6 @@ __global__ void k_paint_table(const tk_draw_record* __restrict__ draws, uint32_t
     out[d] = info;
 }
 
-// extend_coord_i32 (shared/brush/pattern.hlsli:9-17) with
-// euclidean_remainder_i32 (shared/integer.hlsli:5-9).
-__device__ __forceinline__ uint32_t extend_coord(int32_t v, uint32_t size, uint32_t extend) {
-    if (size <= 1u) return 0u;
-    if (extend == TK_EXTEND_REPEAT || extend == TK_EXTEND_REFLECT) {
-        const uint32_t period = size * (extend == TK_EXTEND_REFLECT ? 2u : 1u);
-        const uint32_t mag = v < 0 ? 0u - uint32_t(v) : uint32_t(v), rem = mag % period;
-        const uint32_t coord = v < 0 && rem != 0u ? period - rem : rem;
-        return coord < size ? coord : period - coord - 1u;
-    }
-    return uint32_t(min(max(v, 0), int32_t(size) - 1));
-}
-
-// lerp_premul_u8 (shared/pixel.hlsli:55-62): one fused interpolation per channel.
-__device__ __forceinline__ uint32_t lerp_premul_u8(uint32_t a, uint32_t b, float t) {
-    uint32_t out = 0u;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        const float l = float((a >> (8 * c)) & 255u), r = float((b >> (8 * c)) & 255u);
-        out |= f2u(clampf(mad(r - l, t, l) + 0.5f, 0.0f, 255.0f)) << (8 * c);
-    }
-    return out;
-}
-
-// The image pattern decoded in g / k at brush-space point (x, y):
-// pattern_transform_component (shared/pattern_transform.hlsli:7-11) and
-// sample_resource_pattern_texture (shared/brush/texture.hlsli:11-31). Float to
-// integer conversions saturate and take NaN to 0. The bilinear, pad-extended
-// form is the texture unit's filter in the reference (SampleLevel with
-// clamp-to-edge addressing); here it is that filter computed exactly: texel
-// centres at half-integers, f32 weights, one rounding to 8 bits.
-__device__ __noinline__ uint32_t pattern_at(const Paint& P, const float* g, uint4 k, float x, float y) {
-    const float bx = g[8] * y, by = g[9] * y;
-    const float tx = ((mad(g[6], x, bx) + mad(g[8], y, -bx)) + g[10]) * g[12];
-    const float ty = ((mad(g[7], x, by) + mad(g[9], y, -by)) + g[11]) * g[13];
-    const uint32_t w = __float_as_uint(g[14]), h = __float_as_uint(g[15]), extend = k.w;
-    const uint32_t* __restrict__ tex = P.texels + k.y;
-    uint32_t color;
-    if ((k.x & kGradBilinear) && extend == TK_EXTEND_PAD) {
-        const float sx = clampf(tx, 0.0f, g[12]) - 0.5f, sy = clampf(ty, 0.0f, g[13]) - 0.5f;
-        const float fx0 = floorf(sx), fy0 = floorf(sy), fx = sx - fx0, fy = sy - fy0;
-        const int32_t ix = __float2int_rz(fx0), iy = __float2int_rz(fy0);
-        const uint32_t x0 = uint32_t(min(max(ix, 0), int32_t(w) - 1)), x1 = uint32_t(min(max(ix + 1, 0), int32_t(w) - 1));
-        const uint32_t y0 = uint32_t(min(max(iy, 0), int32_t(h) - 1)), y1 = uint32_t(min(max(iy + 1, 0), int32_t(h) - 1));
-        const float4 tl = rgba8_to_unorm(__ldg(tex + uint64_t(y0) * w + x0)), tr = rgba8_to_unorm(__ldg(tex + uint64_t(y0) * w + x1));
-        const float4 bl = rgba8_to_unorm(__ldg(tex + uint64_t(y1) * w + x0)), br = rgba8_to_unorm(__ldg(tex + uint64_t(y1) * w + x1));
-        const float4 top = make_float4(mad(tr.x - tl.x, fx, tl.x), mad(tr.y - tl.y, fx, tl.y), mad(tr.z - tl.z, fx, tl.z),
-                                       mad(tr.w - tl.w, fx, tl.w));
-        const float4 bot = make_float4(mad(br.x - bl.x, fx, bl.x), mad(br.y - bl.y, fx, bl.y), mad(br.z - bl.z, fx, bl.z),
-                                       mad(br.w - bl.w, fx, bl.w));
-        color = unorm_to_rgba8(make_float4(mad(bot.x - top.x, fy, top.x), mad(bot.y - top.y, fy, top.y),
-                                           mad(bot.z - top.z, fy, top.z), mad(bot.w - top.w, fy, top.w)));
-    } else if (k.x & kGradBilinear) {
-        const float sx = tx - 0.5f, sy = ty - 0.5f;
-        const float fx0 = floorf(sx), fy0 = floorf(sy), fx = sx - fx0, fy = sy - fy0;
-        const int32_t ix = __float2int_rz(fx0), iy = __float2int_rz(fy0);
-        const int32_t jx = int32_t(uint32_t(ix) + 1u), jy = int32_t(uint32_t(iy) + 1u);
-        const uint64_t r0 = uint64_t(extend_coord(iy, h, extend)) * w, r1 = uint64_t(extend_coord(jy, h, extend)) * w;
-        const uint32_t c0 = extend_coord(ix, w, extend), c1 = extend_coord(jx, w, extend);
-        const uint32_t top = lerp_premul_u8(__ldg(tex + r0 + c0), __ldg(tex + r0 + c1), fx);
-        const uint32_t bot = lerp_premul_u8(__ldg(tex + r1 + c0), __ldg(tex + r1 + c1), fx);
-        color = lerp_premul_u8(top, bot, fy);
-    } else {
-        const uint32_t c = extend_coord(__float2int_rz(floorf(tx)), w, extend);
-        const uint32_t r = extend_coord(__float2int_rz(floorf(ty)), h, extend);
-        color = __ldg(tex + uint64_t(r) * w + c);
-    }
-    return scale_premul_u8(color, k.z);
-}
-
-// sample_gradient at pixel centre (px, py) for the gradient decoded in slot i.
-// IMG: whether image patterns can occur (only SDF draws carry them).
-template <bool IMG>
-__device__ __forceinline__ uint32_t gradient_at(const FineSmem& S, const Paint& P, uint32_t i, float px, float py) {
-    const float* g = S.gp[i];
-    const uint4 k = S.gk[i];
-    const uint32_t code = k.x & 255u, extend = k.w;
-    if (code == kGradConst) return k.y;
-    const float x = mad(g[0], px, mad(g[2], py, g[4]));
-    const float y = mad(g[1], px, mad(g[3], py, g[5]));
-    if (IMG && code == kGradPattern) return pattern_at(P, g, k, x, y);
-    const float tx = mad(g[6], x, mad(g[8], y, g[10]));
-    const float ty = mad(g[7], x, mad(g[9], y, g[11]));
-    float t = 0.0f;
-    if (code == kGradLinear) {
-        if (k.x & kGradDenOk) t = mad(tx - g[12], g[14], (ty - g[13]) * g[15]) / g[16];
-    } else {
-        const float qx = tx - g[12], qy = ty - g[13];
-        const float b = -2.0f * mad(qx, g[14], mad(qy, g[15], g[16]));
-        const float c = mad(qx, qx, mad(qy, qy, g[17]));
-        const float dr = g[21], sr = g[22];
-        bool has_t = false;
-        if (k.x & kGradASmall) {
-            if (fabsf(b) > RADIAL_QUADRATIC_EPSILON) {
-                const float cand = -c / b;
-                if (mad(cand, dr, sr) >= 0.0f) {
-                    has_t = true;
-                    t = cand;
-                }
-            }
-        } else {
-            const float disc = mad(b, b, g[19] * c);
-            if (disc >= 0.0f) {
-                const float root = sqrtf(disc);
-                const float t0 = (-b - root) / g[20], t1 = (-b + root) / g[20];
-                const bool v0 = mad(t0, dr, sr) >= 0.0f, v1 = mad(t1, dr, sr) >= 0.0f;
-                if (v0) {
-                    has_t = true;
-                    t = v1 ? fmaxf(t0, t1) : t0;
-                } else if (v1) {
-                    has_t = true;
-                    t = t1;
-                }
-            }
-        }
-        if (!has_t) return 0u;
-    }
-    return sample_ramp(P, k.y, k.z, t, extend);
-}
-
 // segment_row_parts (shared/coverage.hlsli:7-24) of staged segment j for
 // tile row `row`, with the slope division done once per segment at staging.
 __device__ __forceinline__ RowParts staged_row_parts(const FineSmem& S, uint32_t j, uint32_t row) {
@@ -327,18 +206,6 @@ __device__ __forceinline__ RowParts staged_row_parts(const FineSmem& S, uint32_t
     const float sx0 = mad(y0 - anchor_y, slope, anchor_x);
     const float sx1 = mad(y1 - anchor_y, slope, anchor_x);
     return {0.0f, dy, fminf(sx0, sx1), fmaxf(sx0, sx1)};
-}
-
-// The rows a segment crosses, i.e. where segment_row_parts gives dy != 0:
-// with lo < hi the segment's y extent, clamp(y - row, 0, 1) differs between
-// its ends exactly for rows floor(lo) .. ceil(hi) - 1 (y - row is exact for y
-// in [row, row + 1], and rounds to the same side of that interval otherwise).
-__device__ __forceinline__ uint32_t crossed_rows(float p0y, float p1y) {
-    const float lo = fminf(p0y, p1y), hi = fmaxf(p0y, p1y);
-    if (!(lo < hi)) return 0u;
-    const int32_t r0 = max(f2i(floorf(lo)), 0), r1 = min(f2i(ceilf(hi)) - 1, int32_t(TK_TILE_SIZE) - 1);
-    if (r1 < r0) return 0u;
-    return ((2u << r1) - 1u) & ~((1u << r0) - 1u);
 }
 
 // Crossing lists and partial products for staged segments [0, total) of the
@@ -479,7 +346,7 @@ __device__ __forceinline__ void paint_fill(const FineSmem& S, const Paint& P, ui
             if (c.w != 0.0f) px = src_over_premul_unorm(px, make_float4(c.x * sc, c.y * sc, c.z * sc, c.w * sc));
         }
     } else {
-        const uint32_t g = gradient_at<IMG>(S, P, i, float(gx) + 0.5f, float(gy) + 0.5f);
+        const uint32_t g = gradient_at<IMG>(S.gp[i], S.gk[i], P, float(gx) + 0.5f, float(gy) + 0.5f);
         if (masked == 255u && premul_u8_is_opaque(g)) px = rgba8_to_unorm(g);
         else px = src_over_premul_unorm(px, scale_premul_u8_to_unorm(g, masked));
     }
@@ -495,7 +362,7 @@ __device__ __noinline__ float4 paint_glyph_fill(const FineSmem& S, const Paint P
                                                 uint32_t gx, uint32_t gy, float4 px) {
     const uint32_t paint = S.paint[i];
     const uint32_t color =
-        paint != kGradient ? paint : gradient_at<IMG>(S, P, i, float(gx) + 0.5f, float(gy) + 0.5f);
+        paint != kGradient ? paint : gradient_at<IMG>(S.gp[i], S.gk[i], P, float(gx) + 0.5f, float(gy) + 0.5f);
     return rgba8_to_unorm(src_over_mask_linear_auto_u8(unorm_to_rgba8(px), color, masked));
 }
 
@@ -531,7 +398,7 @@ __device__ __noinline__ float4 composite_glyphs(const FineSmem& S, const Paint P
         const uint32_t content = im.content;
         auto brush = [&]() {
             const uint32_t paint = S.paint[i];
-            return paint != kGradient ? paint : gradient_at<IMG>(S, P, i, sx, sy);
+            return paint != kGradient ? paint : gradient_at<IMG>(S.gp[i], S.gk[i], P, sx, sy);
         };
         if (content == TK_GLYPH_LINEAR_MASK || content == TK_GLYPH_LINEAR_SUBPIXEL_MASK) {
             const uint32_t color = brush();
@@ -799,7 +666,7 @@ __global__ void __launch_bounds__(kFineThreads, SDF == 2u ? 3 : 4)
                     clip = combine_alpha(clip, alpha);
                 } else if (tag == TK_PTCL_IMAGE && (mode == TK_TILE_KIND_SDF || mode == TK_TILE_KIND_MIXED)) {
                     // analytic tiles (fine/specialized.hlsli:84-90): the sample over the pixel, unscaled
-                    const uint32_t g = gradient_at<true>(S, P, i, float(gx) + 0.5f, float(gy) + 0.5f);
+                    const uint32_t g = gradient_at<true>(S.gp[i], S.gk[i], P, float(gx) + 0.5f, float(gy) + 0.5f);
                     px = premul_u8_is_opaque(g) ? rgba8_to_unorm(g) : src_over_premul_unorm(px, rgba8_to_unorm(g));
                 } else {
                     const uint32_t masked = combine_alpha(alpha, clip);
@@ -911,16 +778,21 @@ void launch_paint_table(const tk_draw_record* draws, uint32_t draw_count, const 
 void launch_fine(const SceneView& s, const PassView& p, uint32_t* target, cudaStream_t st) {
     const uint32_t T = p.tile_list ? p.tile_list_n : (p.scenes ? p.total_tiles : s.tw * s.th);
     if (T == 0) return;
+    // Path-only scenes take the kernel with several pixels per thread. The
+    // others stay here: a pixel's SDF shape or glyphs cost far more than the
+    // record's dispatch, which is all that is shared between a thread's pixels
+    // (4096^2, 50,000 paths: 207 -> 130 ms; 2048^2, 12,500 shapes: 1.62 here,
+    // 1.65 there; 1280x800 glyph runs: 0.32 here, 0.49 ms there).
+    if (!s.text && !s.sdf_words) return launch_fine_paths(s, p, target, T, st);
     static bool configured = false;
     if (!configured) {
-        for (auto k : {k_fine<0u, false>, k_fine<1u, false>, k_fine<2u, false>, k_fine<0u, true>, k_fine<1u, true>,
-                       k_fine<2u, true>})
+        for (auto k : {k_fine<1u, false>, k_fine<2u, false>, k_fine<0u, true>, k_fine<1u, true>, k_fine<2u, true>})
             cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(FineSmem)));
         configured = true;
     }
     if (s.sdf_ext) k_star_table<<<1, 32, 0, st>>>();
     auto kernel = s.text ? (!s.sdf_words ? k_fine<0u, true> : (s.sdf_ext ? k_fine<2u, true> : k_fine<1u, true>))
-                         : (!s.sdf_words ? k_fine<0u, false> : (s.sdf_ext ? k_fine<2u, false> : k_fine<1u, false>));
+                         : (s.sdf_ext ? k_fine<2u, false> : k_fine<1u, false>);
     const GlyphView glyphs{p.glyph_list, s.glyphs, s.glyph_images, s.glyph_texels};
     kernel<<<T, kFineThreads, sizeof(FineSmem), st>>>(p.tiles, p.ptcl, s.segments, s.paints, s.brush, s.brush_words,
                                                       s.texels, s.draws, s.sdf, s.segment_capacity, target, s.width, s.height,

@@ -55,7 +55,7 @@ struct alignas(16) PaintInfo {
     uint32_t sdf;
     uint32_t pad[2];
     uint4 gk;            // kind | flags, ramp word (or colour), ramp length, extend
-    float g[24];         // transforms and brush terms (fine.cu stage_gradient)
+    float g[24];         // transforms and brush terms (fine.cu decode_gradient)
 };
 static_assert(sizeof(PaintInfo) == 128, "two 64-byte halves");
 
@@ -190,6 +190,9 @@ void launch_tile_prefix_on(tk_tile_record* tiles, uint32_t T, unsigned long long
                            uint32_t* total, uint32_t* error, uint32_t poll_limit, uint32_t first_ticket,
                            cudaStream_t st);
 void launch_fine(const SceneView& s, const PassView& p, uint32_t* target, cudaStream_t st);
+// launch_fine's kernel for scenes without SDF records and text (fine_paths.cu),
+// over `tiles` tiles (of the pass's list when it has one).
+void launch_fine_paths(const SceneView& s, const PassView& p, uint32_t* target, uint32_t tiles, cudaStream_t st);
 // The per-draw PaintInfo table of the uploaded draws and brush blob; shadow
 // records start at word sdf_shadow_base of the device SDF buffer.
 // images: per image of the texture table its first texel, width and height.
