@@ -981,6 +981,9 @@ void scan_phase_partial(tk_ctx* c) {
     c->marks.clear();
     c->scan_valid = false;
     const uint32_t n = uint32_t(c->rescan.size());
+    // longest first: the order scan_emit's queue takes them in
+    std::stable_sort(c->rescan.begin(), c->rescan.end(),
+                     [&](uint32_t x, uint32_t y) { return c->h_paths[x].line_count > c->h_paths[y].line_count; });
     upload(c->rescan_list, c->rescan.data(), n, st);
     std::vector<uint8_t> sel(c->path_count, 0u);
     for (uint32_t p : c->rescan) sel[p] = 1u;

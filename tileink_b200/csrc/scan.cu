@@ -11,11 +11,13 @@
 //             writes each item's ranges and cursors from its prefix and does
 //             the row-wise backdrop cumsum as a segmented scan in the same
 //             CTA. No CTA waits on another.
-// scan_emit   (scan/emit.hlsl:14-28, scan/clip.hlsli:10-75): one warp per
-//             path; lanes take 32 consecutive lines, DDA step r is the outer
-//             loop and lanes rank their slots with __match_any_sync, giving a
-//             fixed segment order inside every tile.
+// scan_emit   (scan/emit.hlsl:14-28, scan/clip.hlsli:10-75): groups of 32
+//             consecutive lines of a path, in turn; lanes take the group's
+//             (line, step) pairs and rank their slots with __match_any_sync,
+//             giving a fixed segment order inside every tile.
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 #include "device.cuh"
 #include "kernels.h"
@@ -359,53 +361,198 @@ __global__ void k_path_totals(tk_path_record* paths, uint32_t path_count, const 
 
 // scan_emit (scan/emit.hlsl:14-28) in canonical order: a path's lines in
 // order, each line's DDA steps in order, every emitting step taking the next
-// cursor of its tile. Warps take paths from a queue, longest first (the line
-// counts are heavy-tailed and a path is one warp's sequential work). Per group
-// of 32 lines the warp computes each line's scan geometry, then walks the
-// group's (line, step) pairs 32 at a time, so that lanes do not idle on the
-// group's longest line; pairs that fall in the same tile in one round are
-// ranked by lane, which keeps the canonical order.
+// cursor of its tile. A group is 32 consecutive lines of a path; its (line,
+// step) pairs are walked 32 at a time, so that lanes do not idle on the group's
+// longest line, and pairs of one round in the same tile are ranked by lane.
+//
+// CTAs take paths from a queue, longest first (the line counts are
+// heavy-tailed). Only the cursors order a path's groups, so a long path's groups
+// are dealt out to the CTA's warps: each computes its lines and the tiles of
+// its pairs, waits for the warp before it, takes its slots (the cursors of the
+// path's tiles are kept in shared memory when they fit), lets the next warp on
+// and then clips and stores its segments. One warp per path spent a global
+// cursor round trip and the clipping of every 32 pairs in series: 0.75 -> 0.21
+// ms on 2,500 paths of 1,800 lines, 0.19 -> 0.045 ms on 240 paths of 930.
+// Short paths are taken by single warps, which need no such order.
 constexpr int kEmitThreads = 256;
+constexpr uint32_t kEmitWarps = kEmitThreads / 32;
+constexpr uint32_t kEmitPairs = 128;    // pairs of a group whose slots are held at a time
+constexpr uint32_t kEmitLong = 256;     // lines from which a whole CTA takes a path
+constexpr uint32_t kEmitWindow = 5632;  // cursors kept in shared memory (4 CTAs an SM)
 
+struct EmitGroups {
+    Scan scan[kEmitWarps][32];
+    uint32_t first[kEmitWarps][33];  // exclusive prefix of the lines' step counts
+};
+struct EmitSmem : EmitGroups {
+    uint32_t slot[kEmitWarps][kEmitPairs];  // tile offsets of the pairs, then their slots
+    uint8_t line[kEmitWarps][kEmitPairs];   // the pairs' lines within the group
+    uint32_t ticket;
+    uint32_t cursor[kEmitWindow];
+};
+
+// Scan geometry of a path's lines g .. g + 31 in sc / first; the number of
+// their (line, step) pairs.
+__device__ __forceinline__ uint32_t emit_group(const tk_line* __restrict__ lines, const tk_path_record& p, uint32_t pid,
+                                               uint32_t g, Scan* sc, uint32_t* first, uint32_t* error) {
+    const uint32_t lane = threadIdx.x & 31u, l = g + lane;
+    Scan s;
+    bool ok = false;
+    if (l < p.line_count) {
+        tk_line line = load_line(lines, uint64_t(p.line_start) + l);
+        if (line.path_id != pid) atomicOr(error, ERR_LINE_PATH_MISMATCH);
+        else ok = scan_geometry(line, p, s);
+    }
+    const uint32_t n = ok ? s.imax - s.imin : 0u;
+    uint32_t incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= uint32_t(o)) incl += v;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+    __syncwarp();  // the previous group's readers are done with sc / first
+    if (n) sc[lane] = s;
+    first[lane] = incl - n;
+    if (lane == 31) first[32] = total;
+    __syncwarp();
+    return total;
+}
+
+// The line whose steps hold pair j: the last lane with first <= j.
+__device__ __forceinline__ uint32_t emit_line(const uint32_t* first, uint32_t j) {
+    uint32_t lo = 0, hi = 32;
+    while (hi - lo > 1u) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (first[mid] <= j) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// One DDA step's clipped segment record, stored at `slot`.
+__device__ __forceinline__ SegmentRec emit_record(const Scan& s, uint32_t i, float z, int32_t tx, int32_t ty) {
+    const tk_line_segment seg = clipped_segment(s, i, z, tx, ty);
+    const float delta_y = seg.p1y - seg.p0y;
+    const float slope = delta_y != 0.0f ? (seg.p1x - seg.p0x) / delta_y : 0.0f;
+    return {seg.p0x, seg.p0y, seg.p1x, seg.p1y, seg.y_edge, slope, {0u, 0u}};
+}
+__device__ __forceinline__ void emit_store(const SegmentRec& r, uint32_t slot, SegmentRec* segments, uint64_t capacity,
+                                           uint32_t* error, uint32_t* seg_line, uint32_t line) {
+    if (slot < capacity) {
+        float4* dst = reinterpret_cast<float4*>(segments + slot);
+        dst[0] = make_float4(r.p0x, r.p0y, r.p1x, r.p1y);
+        dst[1] = make_float4(r.y_edge, r.slope, 0.0f, 0.0f);
+        if (seg_line) seg_line[slot] = line;
+    } else {
+        atomicOr(error, ERR_SEGMENT_OVERFLOW);
+    }
+}
+
+// Warp w of the CTA waits for its turn / lets warp w's turn come: named barrier
+// 1 + w joins the two warps.
+__device__ __forceinline__ void turn_wait(uint32_t w) { asm volatile("bar.sync %0, 64;" ::"r"(1u + w) : "memory"); }
+__device__ __forceinline__ void turn_pass(uint32_t w) { asm volatile("bar.arrive %0, 64;" ::"r"(1u + w) : "memory"); }
+
+// LONG: paths of kEmitLong lines or more are taken by a whole CTA. The queue is
+// sorted by decreasing line count, so the first shorter path ends the CTA's long
+// ones. The other instance leaves the window's shared memory to the L1 cache,
+// which its warps' cursors live in.
+template <bool LONG>
 __global__ void __launch_bounds__(kEmitThreads, 4)
     k_scan_emit(const tk_line* __restrict__ lines, const tk_path_record* __restrict__ paths, uint32_t path_count,
                 uint32_t* cursors, SegmentRec* segments, uint64_t capacity, uint32_t* error, uint32_t* seg_line,
                 const uint32_t* __restrict__ order, uint32_t* ticket) {
-    __shared__ Scan s_scan[kEmitThreads / 32][32];
-    __shared__ uint32_t s_first[kEmitThreads / 32][33];  // exclusive prefix of the lines' step counts
+    extern __shared__ __align__(16) unsigned char emit_raw[];
+    using Smem = std::conditional_t<LONG, EmitSmem, EmitGroups>;
+    Smem& S = *reinterpret_cast<Smem*>(emit_raw);
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t lt_mask = (1u << lane) - 1u;
-    Scan* sc = s_scan[warp];
-    uint32_t* first = s_first[warp];
-    for (;;) {
-        uint32_t k = 0;
-        if (lane == 0) k = atomicAdd(ticket, 1u);
-        k = __shfl_sync(0xffffffffu, k, 0);
+    Scan* sc = S.scan[warp];
+    uint32_t* first = S.first[warp];
+    uint32_t k = 0;
+    if constexpr (LONG) {
+        for (;;) {  // long paths, by the whole CTA
+            __syncthreads();
+            if (threadIdx.x == 0) S.ticket = atomicAdd(ticket, 1u);
+            __syncthreads();
+            k = S.ticket;
+            if (k >= path_count) return;
+            const uint32_t pid = order ? __ldg(order + k) : k;
+            const tk_path_record p = load_path(paths, pid);
+            if (p.line_count < kEmitLong) break;
+            const bool window = p.data_len <= kEmitWindow;
+            if (window) {
+                for (uint32_t t = threadIdx.x; t < p.data_len; t += kEmitThreads) S.cursor[t] = cursors[p.data_offset + t];
+                __syncthreads();
+            }
+            uint32_t* const cur = window ? S.cursor : cursors + p.data_offset;
+            uint32_t* const slots = S.slot[warp];
+            uint8_t* const owner = S.line[warp];
+            const uint32_t rounds = (p.line_count + kEmitThreads - 1u) / kEmitThreads;
+            for (uint32_t it = 0; it < rounds; ++it) {
+                const uint32_t g = (it * kEmitWarps + warp) * 32u;
+                const uint32_t total = g < p.line_count ? emit_group(lines, p, pid, g, sc, first, error) : 0u;
+                bool turn = it == 0u && warp == 0u;
+                // pairs b0 .. b0 + kEmitPairs - 1: their tiles, their slots in turn, their
+                // segments; the turn passes with the last of them
+                uint32_t b0 = 0u;
+                do {
+                    const uint32_t count = min(total - b0, kEmitPairs);
+                    for (uint32_t b = lane; b < count; b += 32u) {
+                        const uint32_t j = b0 + b, L = emit_line(first, j);
+                        const Scan& s = sc[L];
+                        const uint32_t i = s.imin + (j - first[L]);
+                        const float z = floorf(s.a * float(i) + s.b);
+                        int32_t tx, ty;
+                        scan_tile(s, i, z, tx, ty);
+                        owner[b] = uint8_t(L);
+                        slots[b] = scan_tile_inside(s, tx, ty) ? scan_tile_offset(s, tx, ty) - p.data_offset : 0xFFFFFFFFu;
+                    }
+                    __syncwarp();
+                    if (!turn) turn_wait(warp);
+                    turn = true;
+                    for (uint32_t b = 0; b < count; b += 32u) {
+                        const uint32_t off = b + lane < count ? slots[b + lane] : 0xFFFFFFFFu;
+                        const uint32_t same = __match_any_sync(0xffffffffu, off);
+                        uint32_t base = 0u;
+                        if (off != 0xFFFFFFFFu) base = cur[off];
+                        __syncwarp();
+                        if (off != 0xFFFFFFFFu) {
+                            if (lane == __ffs(same) - 1u) cur[off] = base + __popc(same);
+                            slots[b + lane] = base + __popc(same & lt_mask);
+                        }
+                        __syncwarp();
+                    }
+                    if (b0 + count >= total && !(it + 1u == rounds && warp == kEmitWarps - 1u))
+                        turn_pass((warp + 1u) % kEmitWarps);
+                    for (uint32_t b = lane; b < count; b += 32u) {
+                        const uint32_t j = b0 + b, L = owner[b];
+                        const Scan& s = sc[L];
+                        const uint32_t i = s.imin + (j - first[L]);
+                        const float z = floorf(s.a * float(i) + s.b);
+                        int32_t tx, ty;
+                        scan_tile(s, i, z, tx, ty);
+                        if (scan_tile_inside(s, tx, ty))
+                            emit_store(emit_record(s, i, z, tx, ty), slots[b], segments, capacity, error, seg_line,
+                                       p.line_start + g + L);
+                    }
+                    __syncwarp();  // slots and owner are read before the next pairs overwrite them
+                    b0 += kEmitPairs;
+                } while (b0 < total);
+            }
+        }
+    }
+    for (bool own = LONG && warp == 0u;; own = false) {  // the others, by single warps; warp 0 has the path that ended the loop
+        if (!own) {
+            if (lane == 0) k = atomicAdd(ticket, 1u);
+            k = __shfl_sync(0xffffffffu, k, 0);
+        }
         if (k >= path_count) break;
         const uint32_t pid = order ? __ldg(order + k) : k;
         const tk_path_record p = load_path(paths, pid);
         for (uint32_t g = 0; g < p.line_count; g += 32u) {
-            const uint32_t l = g + lane;
-            Scan s;
-            bool ok = false;
-            if (l < p.line_count) {
-                tk_line line = load_line(lines, uint64_t(p.line_start) + l);
-                if (line.path_id != pid) atomicOr(error, ERR_LINE_PATH_MISMATCH);
-                else ok = scan_geometry(line, p, s);
-            }
-            const uint32_t n = ok ? s.imax - s.imin : 0u;
-            uint32_t incl = n;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= uint32_t(o)) incl += v;
-            }
-            const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-            __syncwarp();  // the previous group's readers are done with sc / first
-            if (n) sc[lane] = s;
-            first[lane] = incl - n;
-            if (lane == 31) first[32] = total;
-            __syncwarp();
+            const uint32_t total = emit_group(lines, p, pid, g, sc, first, error);
             for (uint32_t base = 0; base < total; base += 32u) {
                 const uint32_t j = base + lane;
                 bool emitting = false;
@@ -413,14 +560,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4)
                 float z = 0.0f;
                 int32_t tx = 0, ty = 0;
                 if (j < total) {
-                    // the line whose steps hold pair j: the last lane with first <= j
-                    uint32_t lo = 0, hi = 32;
-                    while (hi - lo > 1u) {
-                        const uint32_t mid = (lo + hi) >> 1;
-                        if (first[mid] <= j) lo = mid;
-                        else hi = mid;
-                    }
-                    L = lo;
+                    L = emit_line(first, j);
                     const Scan& sl = sc[L];
                     i = sl.imin + (j - first[L]);
                     z = floorf(sl.a * float(i) + sl.b);
@@ -434,29 +574,15 @@ __global__ void __launch_bounds__(kEmitThreads, 4)
                 // __syncwarp orders the lanes' accesses, so they can be plain
                 // (L1-cached) loads and stores. The cursor load is issued
                 // first and the clipped segment computed while it is in flight.
-                const uint32_t group = __match_any_sync(0xffffffffu, off);
+                const uint32_t same = __match_any_sync(0xffffffffu, off);
                 uint32_t cbase = 0;
                 if (emitting) cbase = cursors[off];
-                tk_line_segment seg{};
-                float slope = 0.0f;
-                if (emitting) {
-                    seg = clipped_segment(sc[L], i, z, tx, ty);
-                    const float delta_y = seg.p1y - seg.p0y;
-                    slope = delta_y != 0.0f ? (seg.p1x - seg.p0x) / delta_y : 0.0f;
-                }
+                SegmentRec seg{};
+                if (emitting) seg = emit_record(sc[L], i, z, tx, ty);
                 __syncwarp();
                 if (emitting) {
-                    const uint32_t leader = __ffs(group) - 1u;
-                    if (lane == leader) cursors[off] = cbase + __popc(group);
-                    const uint32_t slot = cbase + __popc(group & lt_mask);
-                    if (slot < capacity) {
-                        float4* dst = reinterpret_cast<float4*>(segments + slot);
-                        dst[0] = make_float4(seg.p0x, seg.p0y, seg.p1x, seg.p1y);
-                        dst[1] = make_float4(seg.y_edge, slope, 0.0f, 0.0f);
-                        if (seg_line) seg_line[slot] = p.line_start + g + L;
-                    } else {
-                        atomicOr(error, ERR_SEGMENT_OVERFLOW);
-                    }
+                    if (lane == __ffs(same) - 1u) cursors[off] = cbase + __popc(same);
+                    emit_store(seg, cbase + __popc(same & lt_mask), segments, capacity, error, seg_line, p.line_start + g + L);
                 }
                 __syncwarp();
             }
@@ -511,12 +637,36 @@ void launch_scan_count_paths(const SceneView& s, const uint32_t* list, uint32_t 
     k_scan_count_paths<<<n, 256, 0, st>>>(s.lines, s.paths, s.path_count, list, s.backdrops, s.counts);
 }
 
-void launch_scan_emit_paths(const SceneView& s, const uint32_t* list, uint32_t n, cudaStream_t st) {
-    if (n == 0) return;
+namespace {
+
+// Whole CTAs take the long paths while there are few paths for the GPU's 4,736
+// resident warps (6,000 paths: 0.77 against 1.57 ms); beyond that single warps
+// keep it busy (50,000 paths: 7.7 against 10.5 ms; 35,000 paths of a batch: 1.1
+// against 1.5 ms).
+constexpr uint32_t kEmitFewPaths = 4u * 148u * 32u;
+
+template <bool LONG>
+void launch_emit_as(const SceneView& s, const uint32_t* order, uint32_t n, unsigned grid, cudaStream_t st) {
+    constexpr size_t bytes = LONG ? sizeof(EmitSmem) : sizeof(EmitGroups);
+    static bool configured = false;
+    if (!configured) {
+        cudaFuncSetAttribute(k_scan_emit<LONG>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
+        configured = true;
+    }
     cudaMemsetAsync(s.emit_ticket, 0, sizeof(uint32_t), st);
-    k_scan_emit<<<grid_for(uint64_t(n) * 32, kEmitThreads, 148 * 8), kEmitThreads, 0, st>>>(s.lines, s.paths, n, s.cursors, s.segments,
-                                                                        s.segment_capacity, s.error, s.seg_line, list,
-                                                                        s.emit_ticket);
+    k_scan_emit<LONG><<<grid, kEmitThreads, bytes, st>>>(s.lines, s.paths, n, s.cursors, s.segments, s.segment_capacity,
+                                                         s.error, s.seg_line, order, s.emit_ticket);
+}
+
+void launch_emit(const SceneView& s, const uint32_t* order, uint32_t n, cudaStream_t st) {
+    if (n < kEmitFewPaths) launch_emit_as<true>(s, order, n, grid_for(n, 1, 148 * 4), st);
+    else launch_emit_as<false>(s, order, n, grid_for(uint64_t(n) * 32, kEmitThreads, 148 * 8), st);
+}
+
+}  // namespace
+
+void launch_scan_emit_paths(const SceneView& s, const uint32_t* list, uint32_t n, cudaStream_t st) {
+    if (n) launch_emit(s, list, n, st);
 }
 
 void launch_check_path_totals(const SceneView& s, const uint32_t* bumps, const uint32_t* list, uint32_t n,
@@ -526,12 +676,7 @@ void launch_check_path_totals(const SceneView& s, const uint32_t* bumps, const u
 }
 
 void launch_scan_emit(const SceneView& s, cudaStream_t st) {
-    if (s.path_count == 0) return;
-    uint64_t threads = uint64_t(s.path_count) * 32;
-    cudaMemsetAsync(s.emit_ticket, 0, sizeof(uint32_t), st);
-    k_scan_emit<<<grid_for(threads, kEmitThreads, 148 * 8), kEmitThreads, 0, st>>>(s.lines, s.paths, s.path_count, s.cursors,
-                                                                s.segments, s.segment_capacity, s.error, s.seg_line,
-                                                                s.emit_order, s.emit_ticket);
+    if (s.path_count) launch_emit(s, s.emit_order, s.path_count, st);
 }
 
 }  // namespace tk
