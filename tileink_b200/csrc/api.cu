@@ -206,6 +206,7 @@ struct tk_ctx {
     DBuf<tk_segment_range> ranges;
     DBuf<tk::SegmentRec> segments;
     DBuf<tk::PaintInfo> paints;  // per draw, built at upload
+    DBuf<tk::DrawInfo> infos;    // per draw, built at upload
     uint64_t segment_needed = 0;  // device plan: total from the last frame
     DBuf<uint32_t> image, temp, low;  // target, blur temporary, reduced-resolution blur surface
     tk::ProgressiveScratch prog_scratch;  // progressive blur levels (grown on demand)
@@ -654,6 +655,7 @@ tk::SceneView view(tk_ctx* c) {
     s.error = c->misc.ptr;
     s.seg_line = c->want_seg_line ? c->seg_line.ptr : nullptr;
     s.paints = c->paints.ptr;
+    s.infos = c->infos.ptr;
     s.emit_order = c->emit_order.ptr;
     s.emit_ticket = c->misc.ptr + 4;
     return s;
@@ -832,6 +834,8 @@ void do_upload(tk_ctx* c, const tk_scene_desc& scene, const tk_flatten_desc* fl 
                            uint32_t(c->sdf_shadow_base), c->image_tab.ptr, d.image_count, c->paints.ptr, st);
     upload(c->layers, d.layers, d.layer_count, st);
     upload(c->batch_ids, d.draw_batch_ids, d.draw_count, st);
+    c->infos.reserve(d.draw_count);
+    tk::launch_draw_table(view(c), st);
     upload(c->order, d.draw_order, d.draw_order_count, st);
     upload(c->items, c->h_items.data(), c->h_items.size(), st);
     upload_emit_order(c);
@@ -1530,6 +1534,8 @@ void do_batch_upload(tk_ctx* c, const tk_scene_desc* scenes, uint32_t n) {
                            uint32_t(c->sdf_shadow_base), nullptr, 0u, c->paints.ptr, st);
     upload(c->layers, layers.data(), layers.size(), st);
     upload(c->batch_ids, batch_ids.data(), batch_ids.size(), st);
+    c->infos.reserve(draws.size());
+    tk::launch_draw_table(view(c), st);
     upload(c->order, order.data(), order.size(), st);
     rebuild_items(c);
     upload_emit_order(c);
@@ -1661,6 +1667,7 @@ void tk_ctx_destroy(tk_ctx* c) {
     c->d_scenes.release(); c->bin_scene.release(); c->tile_scene.release();
     c->flat.release();
     c->paints.release();
+    c->infos.release();
     c->tile_active.release();
     c->tile_list.release();
     DiffState& D = c->diff;

@@ -6,12 +6,20 @@
 // meets the bin, preserving order.
 //
 // Counting and emission follow coarse_count_bins / coarse_emit_bins
-// (coarse/count.hlsl:48-73, coarse/emit.hlsl:82-142): one thread per tile
-// walks the bin's candidates in painter order. All draw batches of a target
+// (coarse/count.hlsl:48-73, coarse/emit.hlsl:82-142): one warp walks a tile's
+// bin candidates in painter order, 32 at a time, a lane each; ballots and scans
+// give every particle its place in the stream. All draw batches of a target
 // pass are emitted into one merged stream per tile: each batch with particles
 // in the tile contributes TK_PTCL_BATCH_BEGIN{segment_start = batch id,
 // segment_end = record count, color = kind | skip << 3} followed by the
 // reference batch stream without its END; one END closes the tile.
+// What the walk needs of a draw is decoded once per upload (k_draw_table).
+//
+// What bounds it is latency: a candidate's range and backdrop are one load deep,
+// and a lane per candidate keeps 32 of them in flight per tile. One thread per
+// tile left a 640x360 canvas on 24 CTAs of two warps, each candidate ~1,000
+// cycles after the last: 0.14 + 0.12 ms there, 0.026 + 0.019 with warps. Very large
+// canvases keep a thread per tile (k_coarse_tiles).
 #include <cuda_runtime.h>
 
 #include "device.cuh"
@@ -24,22 +32,17 @@ namespace {
 using namespace tkd;
 
 constexpr int kBinSide = 16;
-// Coarse runs one CTA per 8x8-tile quadrant of a bin (four per bin), so that a
-// 4096^2 canvas gives 1024 CTAs instead of 256; each quadrant walks its bin's
-// candidate list.
-constexpr int kQuadSide = 8;
-constexpr int kQuads = (kBinSide / kQuadSide) * (kBinSide / kQuadSide);
-constexpr int kCoarseThreads = kQuadSide * kQuadSide;
+constexpr int kCoarseThreads = 256, kCoarseWarps = kCoarseThreads / 32;
+constexpr int kQuadSide = 8, kQuads = (kBinSide / kQuadSide) * (kBinSide / kQuadSide);
+constexpr int kQuadThreads = kQuadSide * kQuadSide;
+constexpr uint32_t kPrefetchCount = 8, kPrefetchEmit = 4;  // a tile's loads in flight, counting and emitting
+constexpr uint32_t kCandidates = 256;  // staged at a time, one per thread (their numbers are bytes)
 constexpr uint32_t kChunkClassColor = 1u, kChunkClassSdf = 2u, kChunkClassOther = 4u, kChunkClassOccluder = 8u;
-// DrawInfo::meta bits (the draw's batch ordinal above them, from bit kMetaBatchShift)
+// DrawInfo::meta bits (staged candidates: the batch ordinal in the pass above them, from bit kMetaBatchShift)
 constexpr uint32_t kMetaPath = 16u, kMetaSolid = 32u, kMetaSdf = 64u, kMetaSdfSolidClass = 128u, kMetaGlyph = 256u;
 constexpr uint32_t kMetaBatchShift = 9u;
 // DrawInfo::py bits of an SDF draw (px holds its first SDF word)
 constexpr uint32_t kSdfPlain = 256u, kSdfIdentity = 512u, kSdfImage = 1024u;
-// Candidates whose tile loads are in flight together, per pass (emission
-// keeps more state live and holds fewer).
-constexpr uint32_t kPrefetchCount = 8, kPrefetchEmit = 4;
-
 __device__ __forceinline__ uint32_t tile_min_(int32_t px, uint32_t lim) {
     return px > 0 ? min(uint32_t(px) / TK_TILE_SIZE, lim) : 0u;
 }
@@ -51,7 +54,7 @@ __device__ __forceinline__ uint32_t tile_max_(int32_t px, uint32_t lim) {
 // Binning.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-    k_bins(const tk_draw_record* __restrict__ draws, const uint32_t* __restrict__ order, uint32_t order0,
+    k_bins(const DrawInfo* __restrict__ info, const uint32_t* __restrict__ order, uint32_t order0,
            uint32_t draw_n, uint32_t tw, uint32_t th, uint32_t nbx, uint32_t* bin_lists, uint32_t* bin_counts,
            const BatchScene* __restrict__ scenes, const uint32_t* __restrict__ bin_scene) {
     __shared__ uint32_t s_warp[8];
@@ -81,9 +84,8 @@ __global__ void __launch_bounds__(256)
         uint32_t d = 0;
         if (j < draw_n) {
             d = __ldg(order + order0 + j);
-            const tk_pixel_bounds pb = draws[d].pixel_bounds;
-            uint32_t x0 = tile_min_(pb.x0, tw), y0 = tile_min_(pb.y0, th);
-            uint32_t x1 = tile_max_(pb.x1, tw), y1 = tile_max_(pb.y1, th);
+            const uint2 t = *reinterpret_cast<const uint2*>(&info[d].tx);
+            const uint32_t x0 = t.x & 0xFFFFu, x1 = t.x >> 16, y0 = t.y & 0xFFFFu, y1 = t.y >> 16;
             hit = x0 < x1 && y0 < y1 && x0 < bx1 && x1 > bx0 && y0 < by1 && y1 > by0;
         }
         uint32_t ballot = __ballot_sync(0xffffffffu, hit);
@@ -106,15 +108,6 @@ __global__ void __launch_bounds__(256)
 // ---------------------------------------------------------------------------
 // Coarse count / emit.
 // ---------------------------------------------------------------------------
-struct DrawInfo {
-    uint32_t draw;
-    uint32_t tx, ty;         // draw tile bbox: x0 | x1 << 16, y0 | y1 << 16
-    uint32_t px, py;         // path tile bbox packed the same way; SDF draws: first SDF word, kind | flags
-    uint32_t data_offset;
-    uint32_t meta;           // tag | fill << 3 | kMeta* bits | batch << kMetaBatchShift
-    uint32_t color;
-};
-
 struct Ctx {
     const tk_draw_record* draws;
     const tk_path_record* paths;
@@ -319,19 +312,95 @@ static __device__ __noinline__ uint32_t sdf_particle(const tk_draw_record* draws
     return (meta & kMetaSolid) ? TK_PTCL_COLOR : TK_PTCL_IMAGE;
 }
 
+// What binning and the candidate walk need of draw `di` (struct DrawInfo).
+__global__ void k_draw_table(Ctx c, uint32_t draw_count, const uint32_t* __restrict__ batch_ids, DrawInfo* out) {
+    const uint32_t di = blockIdx.x * blockDim.x + threadIdx.x;
+    if (di >= draw_count) return;
+    const tk_draw_record& d = c.draws[di];
+    DrawInfo info{};
+    info.batch = batch_ids[di];
+    info.tx = tile_min_(d.pixel_bounds.x0, 65535u) | (tile_max_(d.pixel_bounds.x1, 65535u) << 16);
+    info.ty = tile_min_(d.pixel_bounds.y0, 65535u) | (tile_max_(d.pixel_bounds.y1, 65535u) << 16);
+    bool valid_path = d.path_id != TK_INVALID_INDEX && d.tag <= TK_DRAW_PATH_GLYPH && d.path_id < c.path_count;
+    if (valid_path) {
+        const tk_path_record& p = c.paths[d.path_id];
+        info.px = p.tile_x0 | (p.tile_x1 << 16);
+        info.py = p.tile_y0 | (p.tile_y1 << 16);
+        info.data_offset = p.data_offset;
+    }
+    bool color_candidate = false;
+    info.color = di;
+    // nontransparent_solid (coarse/paint.hlsli:13-17)
+    const bool solid = d.brush_offset != TK_INVALID_INDEX && brush_word(c, d.brush_offset) == TK_BRUSH_SOLID &&
+                       brush_word(c, d.brush_offset + TK_BRUSH_COLOR_WORD) != 0u;
+    // a glyph run draw gives a PTCL_GLYPH particle or none
+    // (coarse/emit_draw.hlsli:15-22)
+    const bool glyph = c.glyph_runs && d.glyph_run_id != TK_INVALID_INDEX;
+    const bool has_sdf = !glyph && (d.sdf_offset != TK_INVALID_INDEX || d.sdf_shadow_offset != TK_INVALID_INDEX);
+    uint32_t bits = 0u;
+    if (glyph) {
+        valid_path = false;
+        if (d.tag == TK_DRAW_BRUSH && d.glyph_run_id < c.glyph_run_count) {
+            const tk_glyph_run run = c.glyph_runs[d.glyph_run_id];
+            info.px = run.first;
+            info.py = run.count;
+            bits |= kMetaGlyph;
+        }
+    } else if (has_sdf) {
+        // draw_has_sdf (shared/draw.hlsli:31): only brush draws give a particle
+        valid_path = false;
+        const bool plain = d.sdf_offset != TK_INVALID_INDEX;
+        info.px = plain ? d.sdf_offset : uint32_t(c.sdf_shadow_base) + d.sdf_shadow_offset;
+        const uint32_t kind = __ldg(c.sdf + info.px);
+        const bool ident = d.transform.a == 1.0f && d.transform.b == 0.0f && d.transform.c == 0.0f &&
+                           d.transform.d == 1.0f;
+        // full_tile_image's brush test: an image pattern at full opacity
+        const bool image = d.brush_offset != TK_INVALID_INDEX &&
+                           brush_word(c, d.brush_offset) == TK_BRUSH_PATTERN_RESOURCE &&
+                           brush_word(c, d.brush_offset + TK_BRUSH_IMAGE_ALPHA_WORD) == 255u;
+        info.py = (kind & 255u) | (plain ? kSdfPlain : 0u) | (ident ? kSdfIdentity : 0u) | (image ? kSdfImage : 0u);
+        if (d.tag == TK_DRAW_BRUSH) bits |= kMetaSdf;
+        if (solid) {
+            color_candidate = true;
+            info.color = brush_word(c, d.brush_offset + TK_BRUSH_COLOR_WORD);
+        }
+        // solid_supported_sdf (coarse/paint.hlsli:21-25)
+        if (solid && plain && (kind == TK_SDF_RECT || kind == TK_SDF_CANDLESTICK || kind == TK_SDF_CHECKERBOARD))
+            bits |= kMetaSdfSolidClass;
+    } else if (d.tag == TK_DRAW_BRUSH && d.solid_rect != 0u && d.transform.b == 0.0f && d.transform.c == 0.0f && solid) {
+        color_candidate = true;
+        info.color = brush_word(c, d.brush_offset + TK_BRUSH_COLOR_WORD);
+    }
+    if (d.tag == TK_DRAW_CLIP) info.color = 0u;
+    const uint32_t rule = has_sdf ? 0u : (d.fill_rule & 1u);  // SDF particles carry rule 0
+    info.meta = (d.tag & 7u) | (rule << 3) | (valid_path ? kMetaPath : 0u) | (color_candidate ? kMetaSolid : 0u) | bits;
+    out[di] = info;
+}
+
+// A tile's stream between candidate steps. `wrappers` is TK_INVALID_INDEX for a
+// rejected batch, and `batch` for none yet.
+struct TileState {
+    uint64_t at, section;           // emission: next record; the open batch's BATCH_BEGIN
+    uint32_t batch, wrappers, nb, flags;
+    uint32_t glyphs;                // emission: next glyph of the list
+};
+
 // SDF: whether the scene has SDF records; path-only scenes run the instance
 // without the SDF candidate handling. TEXT: whether it has glyph runs; the
 // glyph particle handling (and its calls) lives only in those instances.
 template <bool EMIT, bool SDF, bool TEXT>
 __global__ void __launch_bounds__(kCoarseThreads)
-    k_coarse(Ctx c, const uint32_t* __restrict__ bin_lists, const uint32_t* __restrict__ bin_counts, uint32_t draw_n,
-             uint32_t nbx, const uint32_t* __restrict__ batch_ids, const PassBatch* __restrict__ batches,
-             uint32_t batch0, tk_tile_record* tiles, tk_ptcl_record* ptcl, uint64_t cap,
-             unsigned long long* stats, uint32_t* error, const BatchScene* __restrict__ scenes,
+    k_coarse(Ctx c, const DrawInfo* __restrict__ infos, const uint32_t* __restrict__ bin_lists,
+             const uint32_t* __restrict__ bin_counts, uint32_t draw_n, uint32_t nbx,
+             const PassBatch* __restrict__ batches, uint32_t batch0, tk_tile_record* tiles, tk_ptcl_record* ptcl,
+             uint64_t cap, unsigned long long* stats, uint32_t* error, const BatchScene* __restrict__ scenes,
              const uint32_t* __restrict__ bin_scene, const uint8_t* __restrict__ tile_active, uint32_t* glyph_list,
              uint64_t glyph_cap) {
-    __shared__ DrawInfo s_d[kCoarseThreads];
-    const uint32_t bin = blockIdx.x / kQuads, quad = blockIdx.x % kQuads;
+    constexpr uint32_t kGroups = kBinSide * kBinSide / kCoarseWarps;  // CTAs per bin: half a row of tiles each
+    __shared__ DrawInfo s_d[kCandidates];
+    __shared__ uint32_t s_draw[kCandidates];
+    __shared__ uint8_t s_hit[kCoarseWarps][kCandidates];
+    const uint32_t bin = blockIdx.x / kGroups, group = blockIdx.x % kGroups;
     uint32_t lbin = bin, tile_base = 0u;
     uint64_t list_at = uint64_t(bin) * draw_n;
     if (scenes) {  // batched pass: this bin's canvas
@@ -344,11 +413,302 @@ __global__ void __launch_bounds__(kCoarseThreads)
         tile_base = sc.tile_base;
         list_at = sc.list_base + uint64_t(lbin) * sc.draw_n;
     }
-    const uint32_t qx = quad % (kBinSide / kQuadSide), qy = quad / (kBinSide / kQuadSide);
-    const uint32_t tx = (lbin % nbx) * kBinSide + qx * kQuadSide + (threadIdx.x % kQuadSide);
-    const uint32_t ty = (lbin / nbx) * kBinSide + qy * kQuadSide + (threadIdx.x / kQuadSide);
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t lt = (1u << lane) - 1u;
+    const uint32_t tx = (lbin % nbx) * kBinSide + (group & 1u) * kCoarseWarps + warp;
+    const uint32_t ty = (lbin / nbx) * kBinSide + (group >> 1), tile = tile_base + ty * c.tw + tx;
     const bool in_canvas = tx < c.tw && ty < c.th;
-    const uint32_t tile = tile_base + ty * c.tw + tx;
+    // incremental render: tiles that are not redrawn get no particles
+    const bool live = in_canvas && (!tile_active || tile_active[tile]);
+    if (!EMIT && in_canvas && !live && lane == 0u) {
+        tiles[tile].ptcl_count = 0u;
+        tiles[tile].glyph_count = 0u;
+    }
+    if (!__syncthreads_or(live)) return;
+    TileState st{0u, 0u, TK_INVALID_INDEX, TK_INVALID_INDEX, 0u, 0u, 0u};
+    if (EMIT && live) {
+        st.at = tiles[tile].ptcl_start;
+        if (TEXT) st.glyphs = tiles[tile].glyph_start;
+    }
+    uint32_t lane_total = 0u, lane_glyphs = 0u;
+    const uint32_t* list = bin_lists + list_at;
+    const uint32_t n = bin_counts[bin];
+    unsigned long long fills = 0, visits = 0;
+
+    // A batch's BATCH_BEGIN, once its `nb` particles and its stack's ends (up to
+    // `end`) are stored.
+    const auto store_header = [&](const PassBatch& b, uint64_t section, uint64_t end, uint32_t nb, uint32_t wrappers,
+                                  uint32_t flags) {
+        uint32_t skip = 0;
+        if ((flags & kChunkClassOccluder) && !wrappers) skip = occluded_prefix_g(ptcl, section + 1u, end);
+        // classify_tile_flags (coarse/tile_classification.hlsli:6-10)
+        uint32_t kind = TK_TILE_KIND_EMPTY;
+        if (flags & kChunkClassOther) kind = TK_TILE_KIND_INTERPRETER;
+        else if (flags & kChunkClassSdf) kind = (flags & kChunkClassColor) ? TK_TILE_KIND_MIXED : TK_TILE_KIND_SDF;
+        else if (flags & kChunkClassColor) kind = TK_TILE_KIND_COLOR;
+        store_ptcl(ptcl, cap, section, TK_PTCL_BATCH_BEGIN, 0u, 0u, b.batch_id, nb + 2u * wrappers,
+                   kind | (skip << TK_TILE_PREFIX_SHIFT), error);
+    };
+
+    for (uint32_t c0 = 0; c0 < n; c0 += kCandidates) {
+        __syncthreads();
+        const uint32_t m = min(kCandidates, n - c0);
+        if (threadIdx.x < m) {
+            const uint32_t di = list[c0 + threadIdx.x];
+            DrawInfo info = infos[di];
+            info.meta |= (info.batch - batch0) << kMetaBatchShift;
+            s_d[threadIdx.x] = info;
+            s_draw[threadIdx.x] = di;
+        }
+        __syncthreads();
+        if (!live) continue;
+        // the candidates whose tile boxes hold the tile, in order: a quarter of the
+        // bin's, so that the steps below run with full warps
+        uint32_t hits = 0u;
+        uint8_t* const hit_list = s_hit[warp];
+#pragma unroll 1
+        for (uint32_t k0 = 0; k0 < m; k0 += 32u) {
+            const uint32_t k = k0 + lane;
+            bool in = false;
+            if (k < m) {
+                const DrawInfo& d = s_d[k];
+                const uint32_t tag = d.meta & 7u;
+                in = tx >= (d.tx & 0xFFFFu) && tx < (d.tx >> 16) && ty >= (d.ty & 0xFFFFu) && ty < (d.ty >> 16);
+                if (!(SDF && (d.meta & kMetaSdf)) && !(TEXT && (d.meta & kMetaGlyph)))
+                    in = in && (d.meta & kMetaPath) && tx >= (d.px & 0xFFFFu) && tx < (d.px >> 16) &&
+                         ty >= (d.py & 0xFFFFu) && ty < (d.py >> 16) &&
+                         (tag == TK_DRAW_BRUSH || tag == TK_DRAW_PATH_GLYPH || tag == TK_DRAW_CLIP);
+            }
+            const uint32_t mask = __ballot_sync(0xffffffffu, in);
+            if (in) hit_list[hits + __popc(mask & lt)] = uint8_t(k);
+            hits += __popc(mask);
+        }
+        __syncwarp();
+        // a hit's range and backdrop are loaded a step ahead
+        const auto fetch = [&](uint32_t h, uint32_t& k, tk_segment_range& r, uint32_t& w) {
+            // 0: none, 1: path, 2: SDF, 3: glyphs
+            r = tk_segment_range{0u, 0u};
+            w = k = 0u;
+            if (h >= hits) return 0u;
+            k = hit_list[h];
+            const DrawInfo& d = s_d[k];
+            if (SDF && (d.meta & kMetaSdf)) return 2u;
+            if (TEXT && (d.meta & kMetaGlyph)) return 3u;
+            const uint32_t px0 = d.px & 0xFFFFu, px1 = d.px >> 16, py0 = d.py & 0xFFFFu;
+            const uint32_t bd = d.data_offset + (ty - py0) * (px1 - px0) + tx - px0;
+            r = c.ranges[bd];
+            w = uint32_t(c.backdrops[bd]);
+            return 1u;
+        };
+        tk_segment_range r1;
+        uint32_t w1, k1, hit1 = fetch(lane, k1, r1, w1);
+#pragma unroll 1
+        for (uint32_t h0 = 0; h0 < hits; h0 += 32u) {
+            tk_segment_range r = r1;
+            const uint32_t w = w1, hit = hit1, k = k1;
+            hit1 = fetch(h0 + 32u + lane, k1, r1, w1);
+            uint32_t ptag = 0u, glyphs_here = 0u;  // ptag 0: no particle
+            if (hit) {
+                const DrawInfo& d = s_d[k];
+                const uint32_t tag = d.meta & 7u;
+                ptag = TK_PTCL_FILL;
+                if (TEXT && hit == 3u) {
+                    glyphs_here = draw_glyphs(c, s_draw[k], d.px, d.py, tx, ty, nullptr, 0u, 0u, error);
+                    ptag = glyphs_here ? TK_PTCL_GLYPH : 0u;
+                } else if (SDF && hit == 2u) {
+                    ptag = sdf_particle(c.draws, c.sdf, s_draw[k], d.px, d.py, d.meta, tx, ty);
+                    // an SDF particle names its draw in segment_start (coarse/emit_draw.hlsli:28)
+                    if (ptag == TK_PTCL_SDF) r.start = s_draw[k];
+                } else if (r.start == r.end && w == 0u) {
+                    ptag = 0u;
+                } else if (tag == TK_DRAW_CLIP) {
+                    ptag = TK_PTCL_BEGIN_CLIP;
+                } else if (tag == TK_DRAW_PATH_GLYPH) {
+                    ptag = TK_PTCL_PATH_GLYPH;
+                } else if ((d.meta & kMetaSolid) && r.start == r.end) {
+                    ptag = TK_PTCL_COLOR;
+                }
+            }
+            const uint32_t some = __ballot_sync(0xffffffffu, ptag != 0u);
+            if (!some) continue;
+            // batch starts: particles of another batch than the particle before
+            const uint32_t meta = ptag ? s_d[k].meta : 0u, batch = meta >> kMetaBatchShift;
+            const uint32_t before = some & lt;
+            const uint32_t prev = __shfl_sync(0xffffffffu, batch, before ? 31 - __clz(before) : 0);
+            const bool starts = ptag && batch != (before ? prev : st.batch);
+            const uint32_t start_mask = __ballot_sync(0xffffffffu, starts);
+            uint32_t wrappers = st.wrappers;
+            uint32_t from = 0u;  // the particle's batch start in this step, 32: before the step
+            if (start_mask) {
+                if (starts) wrappers = stack_wrappers<SDF>(c, batches[batch], tx, ty);
+                const uint32_t upto = start_mask & (lt | (1u << lane));
+                from = upto ? 31u - __clz(upto) : 32u;
+                const uint32_t ws = __shfl_sync(0xffffffffu, wrappers, from & 31u);
+                if (from < 32u) wrappers = ws;
+            } else {
+                from = 32u;
+            }
+            const bool accept = ptag && wrappers != TK_INVALID_INDEX;
+            const uint32_t last = 31u - __clz(some);  // the step's last particle
+            if (!EMIT) {
+                lane_total += accept ? 1u : 0u;
+                if (starts && accept) lane_total += 2u * wrappers + 1u;
+                if (accept) lane_glyphs += glyphs_here;
+            } else {
+                const uint32_t accepted = __ballot_sync(0xffffffffu, accept);
+                // the particles of the lane's batch before it in this step
+                const uint32_t since = from < 32u ? ~((1u << from) - 1u) : 0xFFFFFFFFu;
+                const uint32_t nb = __popc(accepted & lt & since) + (from < 32u ? 0u : st.nb);
+                // particle_class_flags (coarse/paint.hlsli:35-40)
+                const uint32_t tag = meta & 7u;
+                uint32_t color = 0u, cls = 0u;
+                if (accept) {
+                    color = ptag == TK_PTCL_COLOR ? s_d[k].color : (tag == TK_DRAW_CLIP ? 0u : s_draw[k]);
+                    cls = kChunkClassOther;
+                    if (ptag == TK_PTCL_COLOR) cls = kChunkClassColor;
+                    else if (ptag == TK_PTCL_IMAGE || (ptag == TK_PTCL_SDF && (meta & kMetaSdfSolidClass)))
+                        cls = kChunkClassSdf;
+                    if (wrappers == 0u && ptag == TK_PTCL_COLOR && (color >> 24) == 255u && nb > 0u)
+                        cls |= kChunkClassOccluder;
+                }
+                // flags of the particles in `lanes`
+                const uint32_t f0 = __ballot_sync(0xffffffffu, cls & kChunkClassColor);
+                const uint32_t f1 = SDF ? __ballot_sync(0xffffffffu, cls & kChunkClassSdf) : 0u;
+                const uint32_t f2 = __ballot_sync(0xffffffffu, cls & kChunkClassOther);
+                const uint32_t f3 = __ballot_sync(0xffffffffu, cls & kChunkClassOccluder);
+                const auto flags_of = [&](uint32_t lanes) {
+                    return (f0 & lanes ? kChunkClassColor : 0u) | (f1 & lanes ? kChunkClassSdf : 0u) |
+                           (f2 & lanes ? kChunkClassOther : 0u) | (f3 & lanes ? kChunkClassOccluder : 0u);
+                };
+                uint64_t at = st.at + __popc(accepted & lt);
+                uint32_t grown = __popc(accepted);
+                // the batch that a start closes: its wrappers, none for a rejected one
+                uint32_t pfrom = 32u, pwr = st.wrappers, extra = 0u;
+                uint64_t section = st.section;
+                if (start_mask) {
+                    const uint32_t pmask = start_mask & lt;
+                    pfrom = pmask ? 31u - __clz(pmask) : 32u;
+                    const uint32_t ws = __shfl_sync(0xffffffffu, wrappers, pfrom & 31u);
+                    if (pfrom < 32u) pwr = ws;
+                    if (starts) extra = (pwr != TK_INVALID_INDEX ? pwr : 0u) + (accept ? 1u + wrappers : 0u);
+                    uint32_t incl = extra;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+                        if (lane >= uint32_t(o)) incl += v;
+                    }
+                    at += incl;
+                    grown += __shfl_sync(0xffffffffu, incl, 31);
+                    if (starts && accept) {
+                        section = at - wrappers - 1u;
+                        emit_stack<SDF>(c, batches[batch], tx, ty, true, ptcl, cap, section + 1u, error);
+                    }
+                }
+                if (TEXT) {
+                    // the tile's glyph list continues at st.glyphs (coarse/emit.hlsl:54-58)
+                    uint32_t incl = accept ? glyphs_here : 0u;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+                        if (lane >= uint32_t(o)) incl += v;
+                    }
+                    if (accept && ptag == TK_PTCL_GLYPH) {
+                        const uint32_t gat = st.glyphs + incl - glyphs_here;
+                        draw_glyphs(c, s_draw[k], s_d[k].px, s_d[k].py, tx, ty, glyph_list, gat, glyph_cap, error);
+                        r = tk_segment_range{gat, gat + glyphs_here};
+                    }
+                    st.glyphs += __shfl_sync(0xffffffffu, incl, 31);
+                }
+                if (accept) {
+                    const bool ranged = ptag != TK_PTCL_COLOR || hit == 1u;
+                    store_ptcl(ptcl, cap, at, ptag, hit == 1u ? w : 0u, ptag == TK_PTCL_GLYPH ? 0u : (meta >> 3) & 1u,
+                               ranged ? r.start : 0u, ranged ? r.end : 0u, color, error);
+                    if (ptag != TK_PTCL_COLOR && ptag != TK_PTCL_SDF && ptag != TK_PTCL_GLYPH) {
+                        fills += 1;
+                        visits += r.end - r.start;
+                    }
+                }
+                if (start_mask) {
+                    // close the batches that end here: their stack's ends, then, with all
+                    // their particles stored, their headers
+                    const uint64_t psection = __shfl_sync(0xffffffffu, section, pfrom & 31u);
+                    const uint32_t pbatch = __shfl_sync(0xffffffffu, batch, pfrom & 31u);
+                    __syncwarp();
+                    if (starts && pwr != TK_INVALID_INDEX) {
+                        const PassBatch& b = batches[pfrom < 32u ? pbatch : st.batch];
+                        const uint64_t end0 = at - (accept ? 1u + wrappers : 0u) - pwr;
+                        const uint64_t end = emit_stack<SDF>(c, b, tx, ty, false, ptcl, cap, end0, error);
+                        const uint32_t lanes = lt & (pfrom < 32u ? ~((1u << pfrom) - 1u) : 0xFFFFFFFFu);
+                        const uint32_t count = __popc(accepted & lanes) + (pfrom < 32u ? 0u : st.nb);
+                        const uint32_t flags = flags_of(lanes) | (pfrom < 32u ? 0u : st.flags) |
+                                               (pwr ? kChunkClassOther : 0u);
+                        store_header(b, pfrom < 32u ? psection : st.section, end, count, pwr, flags);
+                    }
+                    const uint32_t open = 31u - __clz(start_mask), lanes = ~((1u << open) - 1u);
+                    st.section = __shfl_sync(0xffffffffu, section, open);
+                    st.nb = __popc(accepted & lanes);
+                    st.flags = flags_of(lanes);
+                } else {
+                    st.nb += __popc(accepted);
+                    st.flags |= flags_of(0xFFFFFFFFu);
+                }
+                st.at += grown;
+            }
+            if (start_mask) {
+                st.batch = __shfl_sync(0xffffffffu, batch, last);
+                st.wrappers = __shfl_sync(0xffffffffu, wrappers, last);
+            }
+        }
+        __syncwarp();  // the list is read before the next candidates overwrite it
+    }
+    if (live && EMIT) {
+        if (lane == 0u) {
+            uint64_t end = st.at;
+            if (st.batch != TK_INVALID_INDEX && st.wrappers != TK_INVALID_INDEX) {
+                const PassBatch& b = batches[st.batch];
+                end = emit_stack<SDF>(c, b, tx, ty, false, ptcl, cap, end, error);
+                store_header(b, st.section, end, st.nb, st.wrappers, st.flags | (st.wrappers ? kChunkClassOther : 0u));
+            }
+            if (tiles[tile].ptcl_count) store_ptcl(ptcl, cap, end, TK_PTCL_END, 0u, 0u, 0u, 0u, 0u, error);
+        }
+    } else if (live) {
+        const uint32_t total = __reduce_add_sync(0xffffffffu, lane_total);
+        const uint32_t glyphs = TEXT ? __reduce_add_sync(0xffffffffu, lane_glyphs) : 0u;
+        if (lane == 0u) {
+            tiles[tile].ptcl_count = total ? total + 1u : 0u;
+            tiles[tile].glyph_count = glyphs;
+        }
+    }
+    if (EMIT) {
+        for (int o = 16; o > 0; o >>= 1) {
+            fills += __shfl_down_sync(0xffffffffu, fills, o);
+            visits += __shfl_down_sync(0xffffffffu, visits, o);
+        }
+        if (lane == 0u && fills) {
+            atomicAdd(stats + 0, fills);
+            atomicAdd(stats + 1, visits);
+        }
+    }
+}
+
+// The same walk with a thread per tile, one CTA per 8x8-tile quadrant of a bin,
+// for canvases that fill the GPU that way: a warp's 32 neighbouring tiles share
+// most of their candidates and read their ranges side by side.
+template <bool EMIT, bool SDF, bool TEXT>
+__global__ void __launch_bounds__(kQuadThreads)
+    k_coarse_tiles(Ctx c, const DrawInfo* __restrict__ infos, const uint32_t* __restrict__ bin_lists,
+                   const uint32_t* __restrict__ bin_counts, uint32_t draw_n, uint32_t nbx,
+                   const PassBatch* __restrict__ batches, uint32_t batch0, tk_tile_record* tiles, tk_ptcl_record* ptcl,
+                   uint64_t cap, unsigned long long* stats, uint32_t* error, const uint8_t* __restrict__ tile_active,
+                   uint32_t* glyph_list, uint64_t glyph_cap) {
+    __shared__ DrawInfo s_d[kQuadThreads];
+    __shared__ uint32_t s_draw[kQuadThreads];
+    const uint32_t bin = blockIdx.x / kQuads, quad = blockIdx.x % kQuads;
+    const uint32_t qx = quad % (kBinSide / kQuadSide), qy = quad / (kBinSide / kQuadSide);
+    const uint32_t tx = (bin % nbx) * kBinSide + qx * kQuadSide + (threadIdx.x % kQuadSide);
+    const uint32_t ty = (bin / nbx) * kBinSide + qy * kQuadSide + (threadIdx.x / kQuadSide);
+    const bool in_canvas = tx < c.tw && ty < c.th;
+    const uint32_t tile = ty * c.tw + tx;
     // incremental render: tiles that are not redrawn get no particles
     const bool live = in_canvas && (!tile_active || tile_active[tile]);
     if (!__syncthreads_or(live)) {
@@ -358,7 +718,7 @@ __global__ void __launch_bounds__(kCoarseThreads)
         }
         return;
     }
-    const uint32_t* list = bin_lists + list_at;
+    const uint32_t* list = bin_lists + uint64_t(bin) * draw_n;
     const uint32_t n = bin_counts[bin];
 
     uint64_t at = 0, gat = 0;
@@ -391,84 +751,19 @@ __global__ void __launch_bounds__(kCoarseThreads)
         }
     };
 
-    for (uint32_t c0 = 0; c0 < n; c0 += kCoarseThreads) {
+    for (uint32_t c0 = 0; c0 < n; c0 += kQuadThreads) {
         __syncthreads();
         uint32_t j = c0 + threadIdx.x;
         if (j < n) {
-            uint32_t di = list[j];
-            const tk_draw_record& d = c.draws[di];
-            DrawInfo info;
-            info.draw = di;
-            info.tx = tile_min_(d.pixel_bounds.x0, c.tw) | (tile_max_(d.pixel_bounds.x1, c.tw) << 16);
-            info.ty = tile_min_(d.pixel_bounds.y0, c.th) | (tile_max_(d.pixel_bounds.y1, c.th) << 16);
-            bool valid_path = d.path_id != TK_INVALID_INDEX && d.tag <= TK_DRAW_PATH_GLYPH && d.path_id < c.path_count;
-            info.px = 0; info.py = 0; info.data_offset = 0;
-            if (valid_path) {
-                const tk_path_record& p = c.paths[d.path_id];
-                info.px = p.tile_x0 | (p.tile_x1 << 16);
-                info.py = p.tile_y0 | (p.tile_y1 << 16);
-                info.data_offset = p.data_offset;
-            }
-            bool color_candidate = false;
-            info.color = di;
-            // nontransparent_solid (coarse/paint.hlsli:13-17), read only for the
-            // draws that can use it
-            auto solid_paint = [&]() {
-                return d.brush_offset != TK_INVALID_INDEX && brush_word(c, d.brush_offset) == TK_BRUSH_SOLID &&
-                       brush_word(c, d.brush_offset + TK_BRUSH_COLOR_WORD) != 0u;
-            };
-            // a glyph run draw gives a PTCL_GLYPH particle or none
-            // (coarse/emit_draw.hlsli:15-22)
-            const bool glyph = TEXT && c.glyph_runs && d.glyph_run_id != TK_INVALID_INDEX;
-            const bool has_sdf = !glyph && SDF &&
-                                 (d.sdf_offset != TK_INVALID_INDEX || d.sdf_shadow_offset != TK_INVALID_INDEX);
-            uint32_t sdf_bits = 0u;
-            if (glyph) {
-                valid_path = false;
-                if (d.tag == TK_DRAW_BRUSH && d.glyph_run_id < c.glyph_run_count) {
-                    const tk_glyph_run run = c.glyph_runs[d.glyph_run_id];
-                    info.px = run.first;
-                    info.py = run.count;
-                    sdf_bits |= kMetaGlyph;
-                }
-            } else if (has_sdf) {
-                // draw_has_sdf (shared/draw.hlsli:31): only brush draws give a particle
-                valid_path = false;
-                const bool plain = d.sdf_offset != TK_INVALID_INDEX;
-                info.px = plain ? d.sdf_offset : uint32_t(c.sdf_shadow_base) + d.sdf_shadow_offset;
-                const uint32_t kind = __ldg(c.sdf + info.px);
-                const bool ident = d.transform.a == 1.0f && d.transform.b == 0.0f && d.transform.c == 0.0f &&
-                                   d.transform.d == 1.0f;
-                // full_tile_image's brush test: an image pattern at full opacity
-                const bool image = d.brush_offset != TK_INVALID_INDEX &&
-                                   brush_word(c, d.brush_offset) == TK_BRUSH_PATTERN_RESOURCE &&
-                                   brush_word(c, d.brush_offset + TK_BRUSH_IMAGE_ALPHA_WORD) == 255u;
-                info.py = (kind & 255u) | (plain ? kSdfPlain : 0u) | (ident ? kSdfIdentity : 0u) |
-                          (image ? kSdfImage : 0u);
-                if (d.tag == TK_DRAW_BRUSH) sdf_bits |= kMetaSdf;
-                const bool solid = solid_paint();
-                if (solid) {
-                    color_candidate = true;
-                    info.color = brush_word(c, d.brush_offset + TK_BRUSH_COLOR_WORD);
-                }
-                // solid_supported_sdf (coarse/paint.hlsli:21-25)
-                if (solid && plain && (kind == TK_SDF_RECT || kind == TK_SDF_CANDLESTICK || kind == TK_SDF_CHECKERBOARD))
-                    sdf_bits |= kMetaSdfSolidClass;
-            } else if (d.tag == TK_DRAW_BRUSH && d.solid_rect != 0u && d.transform.b == 0.0f &&
-                       d.transform.c == 0.0f && solid_paint()) {
-                color_candidate = true;
-                info.color = brush_word(c, d.brush_offset + TK_BRUSH_COLOR_WORD);
-            }
-            if (d.tag == TK_DRAW_CLIP) info.color = 0u;
-            uint32_t batch = batch_ids[di] - batch0;
-            const uint32_t rule = has_sdf ? 0u : (d.fill_rule & 1u);  // SDF particles carry rule 0
-            info.meta = (d.tag & 7u) | (rule << 3) | (valid_path ? kMetaPath : 0u) |
-                        (color_candidate ? kMetaSolid : 0u) | sdf_bits | (batch << kMetaBatchShift);
+            const uint32_t di = list[j];
+            DrawInfo info = infos[di];
+            info.meta |= (info.batch - batch0) << kMetaBatchShift;
             s_d[threadIdx.x] = info;
+            s_draw[threadIdx.x] = di;
         }
         __syncthreads();
         if (!live) continue;
-        uint32_t m = min(uint32_t(kCoarseThreads), n - c0);
+        uint32_t m = min(uint32_t(kQuadThreads), n - c0);
         // Candidates in groups of kPrefetch: the tile tests and the range /
         // backdrop loads of a whole group are issued first, so that their
         // latencies overlap; the group is then walked in painter order.
@@ -514,14 +809,14 @@ __global__ void __launch_bounds__(kCoarseThreads)
                 uint32_t ptag = TK_PTCL_FILL;
                 uint32_t glyphs_here = 0u;
                 if (TEXT && (glyph_hit & (1u << q))) {
-                    glyphs_here = draw_glyphs(c, d.draw, d.px, d.py, tx, ty, nullptr, 0u, 0u, error);
+                    glyphs_here = draw_glyphs(c, s_draw[k0 + q], d.px, d.py, tx, ty, nullptr, 0u, 0u, error);
                     if (glyphs_here == 0u) continue;
                     ptag = TK_PTCL_GLYPH;
                 } else if (SDF && (sdf_hit & (1u << q))) {
-                    ptag = sdf_particle(c.draws, c.sdf, d.draw, d.px, d.py, meta, tx, ty);
+                    ptag = sdf_particle(c.draws, c.sdf, s_draw[k0 + q], d.px, d.py, meta, tx, ty);
                     if (ptag == 0u) continue;
                     // an SDF particle names its draw in segment_start (coarse/emit_draw.hlsli:28)
-                    r = ptag == TK_PTCL_SDF ? tk_segment_range{d.draw, 0u} : tk_segment_range{0u, 0u};
+                    r = ptag == TK_PTCL_SDF ? tk_segment_range{s_draw[k0 + q], 0u} : tk_segment_range{0u, 0u};
                 } else {
                     if (r.start == r.end && w == 0u) continue;
                     if (tag == TK_DRAW_CLIP) ptag = TK_PTCL_BEGIN_CLIP;
@@ -549,11 +844,11 @@ __global__ void __launch_bounds__(kCoarseThreads)
                     else if (ptag == TK_PTCL_IMAGE || (ptag == TK_PTCL_SDF && (meta & kMetaSdfSolidClass)))
                         cls = kChunkClassSdf;
                     flags |= cls;
-                    uint32_t color = ptag == TK_PTCL_COLOR ? d.color : (tag == TK_DRAW_CLIP ? 0u : d.draw);
+                    uint32_t color = ptag == TK_PTCL_COLOR ? d.color : (tag == TK_DRAW_CLIP ? 0u : s_draw[k0 + q]);
                     if (wrappers == 0u && ptag == TK_PTCL_COLOR && (color >> 24) == 255u && nb > 0u) flags |= kChunkClassOccluder;
                     if (TEXT && ptag == TK_PTCL_GLYPH) {
                         // the tile's glyph list continues at gat (coarse/emit.hlsl:54-58)
-                        draw_glyphs(c, d.draw, d.px, d.py, tx, ty, glyph_list, gat, glyph_cap, error);
+                        draw_glyphs(c, s_draw[k0 + q], d.px, d.py, tx, ty, glyph_list, gat, glyph_cap, error);
                         store_ptcl(ptcl, cap, at++, ptag, 0u, 0u, uint32_t(gat), uint32_t(gat + glyphs_here), color,
                                    error);
                         gat += glyphs_here;
@@ -688,27 +983,56 @@ void launch_bins(const SceneView& s, const PassView& p, cudaStream_t st) {
         cudaMemsetAsync(p.bin_counts, 0, sizeof(uint32_t) * nbins, st);
         return;
     }
-    k_bins<<<nbins, 256, 0, st>>>(s.draws, s.order, p.order0, p.draw_n, s.tw, s.th, p.nbx, p.bin_lists, p.bin_counts,
+    k_bins<<<nbins, 256, 0, st>>>(s.infos, s.order, p.order0, p.draw_n, s.tw, s.th, p.nbx, p.bin_lists, p.bin_counts,
                                   p.scenes, p.bin_scene);
 }
 
+namespace {
+
+Ctx coarse_ctx(const SceneView& s) {
+    return Ctx{s.draws, s.paths, s.path_count, s.layers, s.brush, s.brush_words, s.sdf, s.sdf_shadow_base, s.backdrops,
+               s.ranges, s.tw, s.th, s.glyph_runs, s.glyphs, s.glyph_images, s.glyph_run_count};
+}
+
+}  // namespace
+
+void launch_draw_table(const SceneView& s, cudaStream_t st) {
+    if (s.draw_count)
+        k_draw_table<<<(s.draw_count + 127) / 128, 128, 0, st>>>(coarse_ctx(s), s.draw_count, s.batch_ids, s.infos);
+}
+
+// A thread per tile from this many tiles of one canvas on (4096x4096 / 50,000
+// paths, 65,536 tiles: count 4.7, emit 5.8 ms against 4.9 and 8.3 with a warp
+// per tile; 2048x2048 / 6,000 paths, 16,384 tiles: 0.61 and 0.67 against 0.20 and
+// 0.33 ms). A batch's canvases are small bins of few candidates: always warps
+// (96 scenes: 1.36 and 1.15 against 0.58 and 0.63 ms).
+constexpr uint32_t kThreadPerTile = 32768;
+
 void launch_coarse(const SceneView& s, const PassView& p, bool emit, cudaStream_t st) {
-    Ctx c{s.draws, s.paths, s.path_count, s.layers, s.brush, s.brush_words, s.sdf, s.sdf_shadow_base, s.backdrops,
-          s.ranges, s.tw, s.th, s.glyph_runs, s.glyphs, s.glyph_images, s.glyph_run_count};
     const uint32_t nbins = p.scenes ? p.total_bins : p.nbx * p.nby;
     if (nbins == 0) return;
     const bool sdf = s.sdf_words != 0, text = s.glyph_runs != nullptr;
+    if (!p.scenes && s.tw * s.th >= kThreadPerTile) {
+        using Kernel = decltype(&k_coarse_tiles<true, true, true>);
+        const Kernel table[2][2][2] = {
+            {{k_coarse_tiles<false, false, false>, k_coarse_tiles<false, false, true>},
+             {k_coarse_tiles<false, true, false>, k_coarse_tiles<false, true, true>}},
+            {{k_coarse_tiles<true, false, false>, k_coarse_tiles<true, false, true>},
+             {k_coarse_tiles<true, true, false>, k_coarse_tiles<true, true, true>}}};
+        table[emit][sdf][text]<<<nbins * kQuads, kQuadThreads, 0, st>>>(
+            coarse_ctx(s), s.infos, p.bin_lists, p.bin_counts, p.draw_n, p.nbx, p.batches, p.batch0, p.tiles, p.ptcl,
+            p.ptcl_capacity, p.stats, s.error, p.tile_active, p.glyph_list, p.glyph_capacity);
+        return;
+    }
     using Kernel = decltype(&k_coarse<true, true, true>);
     const Kernel table[2][2][2] = {
         {{k_coarse<false, false, false>, k_coarse<false, false, true>},
          {k_coarse<false, true, false>, k_coarse<false, true, true>}},
         {{k_coarse<true, false, false>, k_coarse<true, false, true>},
          {k_coarse<true, true, false>, k_coarse<true, true, true>}}};
-    const Kernel kernel = table[emit][sdf][text];
-    kernel<<<nbins * kQuads, kCoarseThreads, 0, st>>>(c, p.bin_lists, p.bin_counts, p.draw_n, p.nbx, s.batch_ids,
-                                                      p.batches, p.batch0, p.tiles, p.ptcl, p.ptcl_capacity, p.stats,
-                                                      s.error, p.scenes, p.bin_scene, p.tile_active, p.glyph_list,
-                                                      p.glyph_capacity);
+    table[emit][sdf][text]<<<nbins * (kBinSide * kBinSide / kCoarseWarps), kCoarseThreads, 0, st>>>(
+        coarse_ctx(s), s.infos, p.bin_lists, p.bin_counts, p.draw_n, p.nbx, p.batches, p.batch0, p.tiles, p.ptcl,
+        p.ptcl_capacity, p.stats, s.error, p.scenes, p.bin_scene, p.tile_active, p.glyph_list, p.glyph_capacity);
 }
 
 void launch_tile_prefix(const SceneView& s, const PassView& p, cudaStream_t st) {

@@ -59,6 +59,19 @@ struct alignas(16) PaintInfo {
 };
 static_assert(sizeof(PaintInfo) == 128, "two 64-byte halves");
 
+// A draw as binning and coarse need it, decoded once per upload from the draw,
+// its path record and its brush (coarse.cu, k_draw_table).
+struct alignas(16) DrawInfo {
+    uint32_t tx, ty;         // draw tile bbox (not clamped to the canvas): x0 | x1 << 16, y0 | y1 << 16 (read as a pair)
+    uint32_t px, py;         // path tile bbox packed the same way; SDF draws: first SDF word, kind | flags;
+                             // glyph runs: first glyph, glyphs
+    uint32_t data_offset;    // the path's slice of the pool
+    uint32_t meta;           // tag | fill << 3 | kMeta* bits
+    uint32_t color;
+    uint32_t batch;          // its batch id
+};
+static_assert(sizeof(DrawInfo) == 32, "one sector per draw");
+
 struct SceneView {
     const tk_line* lines;
     uint64_t line_count;
@@ -96,6 +109,7 @@ struct SceneView {
     uint32_t* error;
     uint32_t* seg_line;  // optional: line index of every emitted segment
     const PaintInfo* paints;     // per draw (launch_paint_table)
+    DrawInfo* infos;             // per draw (launch_draw_table)
     const uint32_t* emit_order;  // paths by decreasing line count (optional)
     uint32_t* emit_ticket;       // path queue of scan_emit
 };
@@ -199,6 +213,10 @@ void launch_fine_paths(const SceneView& s, const PassView& p, uint32_t* target, 
 void launch_paint_table(const tk_draw_record* draws, uint32_t draw_count, const uint32_t* brush,
                         uint64_t brush_words, uint32_t sdf_shadow_base, const uint4* images, uint32_t image_count,
                         PaintInfo* out, cudaStream_t st);
+
+// The per-draw DrawInfo table of the uploaded scene (draws, paths, brushes, SDF
+// records, glyph runs and batch ids).
+void launch_draw_table(const SceneView& s, cudaStream_t st);
 
 // Images.
 void launch_fill(uint32_t* image, uint64_t n, uint32_t value, cudaStream_t st);
