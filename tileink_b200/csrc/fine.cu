@@ -781,7 +781,7 @@ void launch_fine(const SceneView& s, const PassView& p, uint32_t* target, cudaSt
     // Path-only scenes take the kernel with several pixels per thread. The
     // others stay here: a pixel's SDF shape or glyphs cost far more than the
     // record's dispatch, which is all that is shared between a thread's pixels
-    // (4096^2, 50,000 paths: 207 -> 130 ms; 2048^2, 12,500 shapes: 1.62 here,
+    // (4096^2, 50,000 paths: 207 -> 128 ms; 2048^2, 12,500 shapes: 1.62 here,
     // 1.65 there; 1280x800 glyph runs: 0.32 here, 0.49 ms there).
     if (!s.text && !s.sdf_words) return launch_fine_paths(s, p, target, T, st);
     static bool configured = false;

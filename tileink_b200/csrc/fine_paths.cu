@@ -7,9 +7,9 @@
 // pixels of a thread, the pixel arithmetic runs on f32 pairs (f32x2), and
 // coverage is evaluated by half rows of fills instead of pixel by pixel.
 // Against one pixel per thread with coverage in the record loop: 4.4 G against
-// 8.5 G warp instructions on the 2048x2048 / 6,000-path frame, 6.3 against
-// 10.1 ms; 4096x4096 / 50,000 paths 130 against 207 ms, 1283x717 / 2,500 paths
-// 1.17 against 1.99 ms, 640x360 / 240 fills 0.27 against 0.29 ms.
+// 8.5 G warp instructions on the 2048x2048 / 6,000-path frame, 6.1 against
+// 10.1 ms; 4096x4096 / 50,000 paths 128 against 207 ms, 1283x717 / 2,500 paths
+// 1.12 against 1.99 ms, 640x360 / 240 fills 0.26 against 0.29 ms.
 // Four pixels per thread (64-thread CTAs) took 6.8 ms on the 2048 frame and
 // eight (one warp a tile) 11.1: too few warps are in flight, and half-size
 // chunks repeat the staging. The loops of the staging are not unrolled and the
@@ -179,25 +179,27 @@ __device__ __forceinline__ void stage_coverage(FineSmem& S, uint32_t& n, uint32_
     // Prefixes over the segments: four words of four row counters (bytes), and
     // one of crossings, product blocks (what a segment can need: one per row and
     // one per group boundary it passes) and left-edge segments, dealt out to the
-    // warps.
+    // warps. A lane takes kPer consecutive segments, so that one warp scan does
+    // (a scan for every 32 segments: 6.3 instead of 6.1 ms on the 2048 frame).
+    constexpr uint32_t kPer = (kSegs + 31u) / 32u;
 #pragma unroll 1
     for (uint32_t t = warp; t < 5u; t += kWarps) {
-        uint32_t carry = 0u;
-#pragma unroll 1
-        for (uint32_t j0 = 0; j0 < total; j0 += 32u) {
-            const uint32_t j = j0 + lane, m = j < total ? S.rmask[j] : 0u;
-            const uint32_t v = t < 4u ? (((m >> (4u * t)) & 15u) * 0x00204081u) & 0x01010101u
-                                      : uint32_t(__popc(m & 0xFFFFu)) * 0x1001u + ((m >> 17) << 12) + ((m & 0x10000u) << 8);
-            const uint32_t incl = warp_inclusive(v, lane);
-            if (j < total) {
-                if (t < 4u) reinterpret_cast<uint32_t*>(&S.pos[j])[t] = carry + incl - v;
-                else S.pre[j] = carry + incl - v;
-            }
-            carry += __shfl_sync(0xffffffffu, incl, 31);
+        uint32_t v[kPer], sum = 0u;
+#pragma unroll
+        for (uint32_t q = 0; q < kPer; ++q) {
+            const uint32_t j = lane * kPer + q, m = j < total ? S.rmask[j] : 0u;
+            v[q] = sum;
+            sum += t < 4u ? (((m >> (4u * t)) & 15u) * 0x00204081u) & 0x01010101u
+                          : uint32_t(__popc(m & 0xFFFFu)) * 0x1001u + ((m >> 17) << 12) + ((m & 0x10000u) << 8);
         }
-        if (lane == 0) {
-            if (t < 4u) reinterpret_cast<uint32_t*>(&S.pos[total])[t] = carry;
-            else S.pre[total] = carry;
+        const uint32_t before_lane = warp_inclusive(sum, lane) - sum;
+#pragma unroll
+        for (uint32_t q = 0; q < kPer; ++q) {
+            const uint32_t j = lane * kPer + q;
+            if (j <= total) {  // the one past the last holds the totals
+                if (t < 4u) reinterpret_cast<uint32_t*>(&S.pos[j])[t] = before_lane + v[q];
+                else S.pre[j] = before_lane + v[q];
+            }
         }
     }
     __syncthreads();
