@@ -18,6 +18,7 @@
 #include "flatten_core.h"
 #include "host.h"
 #include "kernels.h"
+#include "stager.h"
 
 namespace {
 
@@ -235,6 +236,8 @@ struct tk_ctx {
     size_t ev_used = 0;
     std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> marks;
     FlattenScratch flat;
+    std::shared_ptr<tk::Stager> stager;  // large uploads from pageable memory
+    uint64_t large_bytes = 0;            // of such uploads so far
     // incremental rendering: whether `image` holds the last single-scene
     // frame (and its size and clear colour), and the redrawn tiles of the
     // frame in progress (null outside tk_render_incremental)
@@ -294,6 +297,26 @@ template <class T>
 void upload(DBuf<T>& b, const T* src, size_t n, cudaStream_t st) {
     b.reserve(n);
     if (n) TK_CUDA(cudaMemcpyAsync(b.ptr, src, n * sizeof(T), cudaMemcpyHostToDevice, st));
+}
+
+// A copy that may be large, from memory of the caller's.
+void copy_in(tk_ctx* c, void* dst, const void* src, size_t bytes, cudaStream_t st) {
+    if (!bytes) return;
+    if (tk::Stager::wants(src, bytes)) {
+        c->large_bytes += bytes;
+        if (!c->stager && c->large_bytes >= tk::Stager::kPays) c->stager = tk::Stager::of(c->device);
+        const cudaError_t e = c->stager ? c->stager->copy(dst, src, bytes, st) : cudaErrorNotReady;
+        if (e != cudaErrorNotReady) {
+            TK_CUDA(e);
+            return;
+        }
+    }
+    TK_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
+}
+template <class T>
+void upload(tk_ctx* c, DBuf<T>& b, const T* src, size_t n, cudaStream_t st) {
+    b.reserve(n);
+    copy_in(c, b.ptr, src, n * sizeof(T), st);
 }
 
 // Host validation of a scene against the contracts the kernels rely on.
@@ -784,8 +807,8 @@ void do_upload(tk_ctx* c, const tk_scene_desc& scene, const tk_flatten_desc* fl 
     auto side_copies = [&] {
         TK_CUDA(cudaEventRecord(c->ev_main, st));
         TK_CUDA(cudaStreamWaitEvent(cs, c->ev_main, 0));
-        upload(c->draws, d.draws, d.draw_count, cs);
-        upload(c->brush, d.brush_blob, d.brush_word_count, cs);
+        upload(c, c->draws, d.draws, d.draw_count, cs);
+        upload(c, c->brush, d.brush_blob, d.brush_word_count, cs);
         c->sdf.reserve(c->sdf_words);
         if (d.sdf_word_count)
             TK_CUDA(cudaMemcpyAsync(c->sdf.ptr, d.sdf_blob, d.sdf_word_count * 4, cudaMemcpyHostToDevice, cs));
@@ -799,17 +822,16 @@ void do_upload(tk_ctx* c, const tk_scene_desc& scene, const tk_flatten_desc* fl 
         }
         c->texels.reserve(texel_words);
         for (uint32_t k = 0; k < d.image_count; ++k)
-            TK_CUDA(cudaMemcpyAsync(c->texels.ptr + tab[k].x, d.images[k].premul_rgba8,
-                                    uint64_t(tab[k].y) * tab[k].z * 4, cudaMemcpyHostToDevice, cs));
+            copy_in(c, c->texels.ptr + tab[k].x, d.images[k].premul_rgba8, uint64_t(tab[k].y) * tab[k].z * 4, cs);
         upload(c->image_tab, tab.data(), tab.size(), cs);
         upload(c->glyph_runs, d.glyph_runs, d.glyph_run_count, cs);
         upload(c->glyphs, d.glyphs, d.glyph_count, cs);
         upload(c->glyph_images, d.glyph_images, d.glyph_image_count, cs);
-        upload(c->glyph_texels, d.glyph_texels, d.glyph_texel_count, cs);
+        upload(c, c->glyph_texels, d.glyph_texels, d.glyph_texel_count, cs);
         upload(c->filter_words, d.filter_words, d.filter_word_count, cs);
         TK_CUDA(cudaEventRecord(c->ev_copy, cs));
     };
-    upload(c->paths, d.paths, d.path_count, st);
+    upload(c, c->paths, d.paths, d.path_count, st);
     if (fl) {
         flatten_on_device(c, d, *fl, side_copies);  // the host lines, then the device lines
     } else if (line_dirty) {  // the changed paths' line ranges, runs coalesced
@@ -819,13 +841,11 @@ void do_upload(tk_ctx* c, const tk_scene_desc& scene, const tk_flatten_desc* fl 
             uint32_t q = p;
             while (q < d.path_count && (*line_dirty)[q]) ++q;
             const uint64_t a = d.paths[p].line_start, b = uint64_t(d.paths[q - 1].line_start) + d.paths[q - 1].line_count;
-            if (b > a)
-                TK_CUDA(cudaMemcpyAsync(c->lines.ptr + a, d.lines + a, (b - a) * sizeof(tk_line),
-                                        cudaMemcpyHostToDevice, st));
+            if (b > a) copy_in(c, c->lines.ptr + a, d.lines + a, (b - a) * sizeof(tk_line), st);
             p = q;
         }
     } else {
-        upload(c->lines, d.lines, d.line_count, st);
+        upload(c, c->lines, d.lines, d.line_count, st);
     }
     if (!fl) side_copies();
     TK_CUDA(cudaStreamWaitEvent(st, c->ev_copy, 0));
@@ -1291,9 +1311,9 @@ void flatten_on_device(tk_ctx* c, const tk_scene_desc& d, const tk_flatten_desc&
     auto& strokes = F.strokes;
     auto& wide = F.wide;
     auto& pts = F.pts;
-    upload(els, fl.elements, n, st);
+    upload(c, els, fl.elements, n, st);
     upload(path_els, fl.path_elements, 2ull * d.path_count, st);
-    upload(sels, fl.stroke_elements, nse, st);
+    upload(c, sels, fl.stroke_elements, nse, st);
     upload(polys, fl.polylines, npl, st);
     upload(strokes, fl.strokes, ns, st);
     offsets.reserve(n);
@@ -1334,7 +1354,7 @@ void flatten_on_device(tk_ctx* c, const tk_scene_desc& d, const tk_flatten_desc&
     const uint64_t total = host_lines + fill_lines + stroke_lines;
     if (total > 0xFFFFFFFFull) invalid("line count exceeds u32 indexing");
     c->lines.reserve(total);
-    if (host_lines) TK_CUDA(cudaMemcpyAsync(c->lines.ptr, d.lines, host_lines * sizeof(tk_line), cudaMemcpyHostToDevice, st));
+    copy_in(c, c->lines.ptr, d.lines, host_lines * sizeof(tk_line), st);
     tk::launch_flatten_emit(els.ptr, n, offsets.ptr, words.ptr, c->paths.ptr, d.path_count, path_els.ptr, c->lines.ptr,
                             host_lines, host_lines + fill_lines, words.ptr + 1, st);
     tk::launch_stroke_emit(sv, words.ptr + 3, c->paths.ptr, c->lines.ptr, host_lines + fill_lines, total, st);
@@ -1485,9 +1505,7 @@ void do_batch_upload(tk_ctx* c, const tk_scene_desc* scenes, uint32_t n) {
     cudaStream_t st = c->stream;
     c->lines.reserve(total_lines);
     for (uint32_t s = 0; s < n; ++s)
-        if (scenes[s].line_count)
-            TK_CUDA(cudaMemcpyAsync(c->lines.ptr + line_base[s], scenes[s].lines, scenes[s].line_count * sizeof(tk_line),
-                                    cudaMemcpyHostToDevice, st));
+        copy_in(c, c->lines.ptr + line_base[s], scenes[s].lines, scenes[s].line_count * sizeof(tk_line), st);
     DBuf<uint64_t> d_line_base;
     DBuf<uint32_t> d_path_base;
     upload(d_line_base, line_base.data(), line_base.size(), st);
@@ -2321,9 +2339,9 @@ int32_t tk_diff_forward(tk_ctx* c, const tk_diff_scene* sc, const float* target,
         check_error_word(c);
         const uint64_t n = uint64_t(sc->width) * sc->height;
         upload(D.colp, colp.data(), colp.size(), st);
-        upload(D.target, reinterpret_cast<const float4*>(target), n, st);
-        upload(D.ep_point, ep_point.data(), ep_point.size(), st);
-        upload(D.ep_w, ep_w.data(), ep_w.size(), st);
+        upload(c, D.target, reinterpret_cast<const float4*>(target), n, st);
+        upload(c, D.ep_point, ep_point.data(), ep_point.size(), st);
+        upload(c, D.ep_w, ep_w.data(), ep_w.size(), st);
         D.layer.reserve(n);
         D.gI.reserve(n);
         D.sums.reserve(2);
