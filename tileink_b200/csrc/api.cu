@@ -150,7 +150,8 @@ struct DiffState {
     float4 bg{};
     std::vector<float> colors;  // straight RGBA per path
     DBuf<float4> colp, target, layer, t1, blurred, gI, d0, d1;
-    DBuf<float2> scratch, line_acc;
+    DBuf<float> scratch;
+    DBuf<float2> line_acc;
     DBuf<float> color_acc, dpoints, taps, dtaps, ep_w;
     DBuf<uint32_t> ep_point;
     DBuf<double> sums;  // [0] loss [1] dL/dsigma
@@ -2412,7 +2413,6 @@ int32_t tk_diff_backward(tk_ctx* c, float* d_points, float* d_colors, float* d_s
         D.line_acc.reserve(D.lines);
         D.color_acc.reserve(5ull * c->draw_count);
         D.dpoints.reserve(2ull * D.points);
-        D.scratch.reserve(std::max<uint64_t>(p.ptcl_used, 1) * 256);
         TK_CUDA(cudaMemsetAsync(D.sums.ptr + 1, 0, sizeof(double), st));
         TK_CUDA(cudaMemsetAsync(D.line_acc.ptr, 0, std::max<uint64_t>(D.lines, 1) * sizeof(float2), st));
         TK_CUDA(cudaMemsetAsync(D.color_acc.ptr, 0, 5ull * std::max(c->draw_count, 1u) * sizeof(float), st));
@@ -2431,6 +2431,7 @@ int32_t tk_diff_backward(tk_ctx* c, float* d_points, float* d_colors, float* d_s
         }
         tk::SceneView s = view(c);
         tk::PassView v = pass_view(c, p);
+        D.scratch.reserve(tk::diff_scratch_len(p.ptcl_used, uint64_t(s.tw) * s.th));
         tk::launch_diff_fine_bwd(s, v, c->seg_line.ptr, D.colp.ptr, dL, D.scratch.ptr, D.line_acc.ptr,
                                  D.color_acc.ptr, st);
         tk::launch_diff_lines_to_points(c->lines.ptr, D.line_acc.ptr, D.ep_point.ptr, D.ep_w.ptr, D.lines,

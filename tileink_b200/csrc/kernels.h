@@ -322,6 +322,11 @@ void launch_stroke_emit(const StrokeView& v, const uint32_t* line_total, tk_path
                         uint64_t line_base, uint64_t line_end, cudaStream_t st);
 
 // Differentiable rendering (diff.cu): float forward and adjoint.
+constexpr uint32_t kDiffChunk = 16;  // records of a tile walked at a time
+// launch_diff_fine_bwd's scratch, in floats.
+constexpr uint64_t diff_scratch_len(uint64_t ptcl_used, uint64_t tiles) {
+    return (ptcl_used / kDiffChunk + tiles + 1u) * TK_TILE_SIZE * TK_TILE_SIZE;
+}
 void launch_diff_fine_fwd(const SceneView& s, const PassView& p, const float4* colp, float4* layer, cudaStream_t st);
 void launch_diff_blur(const float4* in, float4* out, const float* w, int32_t r, uint32_t width, uint32_t height,
                       int32_t axis, cudaStream_t st);
@@ -332,7 +337,7 @@ void launch_diff_blur_bwd(const float4* dout_src, const float4* fwd_in, float4* 
                           double* sig, cudaStream_t st);
 void launch_diff_composite_bwd(const float4* gI, float4 bg, uint64_t n, float4* dL, cudaStream_t st);
 void launch_diff_fine_bwd(const SceneView& s, const PassView& p, const uint32_t* seg_line, const float4* colp,
-                          const float4* dlayer, float2* scratch, float2* line_acc, float* color_acc, cudaStream_t st);
+                          const float4* dlayer, float* scratch, float2* line_acc, float* color_acc, cudaStream_t st);
 void launch_diff_lines_to_points(const tk_line* lines, const float2* line_acc, const uint32_t* ep_base,
                                  const float* ep_w, uint64_t n, float* dpoints, cudaStream_t st);
 
