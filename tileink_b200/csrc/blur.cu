@@ -237,7 +237,7 @@ __device__ __forceinline__ void acc_pair(Texel& acc, const Texel& a, const Texel
 // neighbouring pixels, which share a texel of three per side and pair, and the third
 // is the next pair's first. Texels outside `bounds` are zero in the tile, which adds
 // what a skipped tap adds.
-// A 1024x1024 frame with a blur of sigma 14 (radius 42) and one of 7 (21): 1.80 ms
+// A 1024x1024 frame with a blur of sigma 14 (radius 42) and one of 7 (21): 1.86 ms
 // with the kernel above (bound by its loads and 16 divisions a sample), 0.63 now. The
 // limit is the tile's shared memory: 17 KB at radius 48.
 template <int AXIS>
