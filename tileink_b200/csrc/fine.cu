@@ -426,8 +426,9 @@ __device__ __noinline__ float4 composite_glyphs(const FineSmem& S, const Paint P
 
 // SDF: 0 for scenes without SDF records, 1 with SDF records of the base
 // kinds, 2 with the extended kinds (candlestick, dash line, triangle,
-// checkerboard). Path-only scenes run the instance without the PTCL_SDF
-// branch, which costs the record loop about 3% even when never taken; the
+// checkerboard). Text scenes without SDF records run the instance without the
+// PTCL_SDF branch, which costs the record loop about 3% even when never taken;
+// scenes of paths alone have a kernel of their own (fine_paths.cu). The
 // extended kinds' code costs the base kinds more, so it has its own instance,
 // with the registers of 3 CTAs per SM.
 // TEXT: the scene has glyph outline fills or glyph runs; their compositing
