@@ -6,7 +6,7 @@
 // serial chain. A record's dispatch and staging are the same for the two
 // pixels of a thread, the pixel arithmetic runs on f32 pairs (f32x2), and
 // coverage is evaluated by half rows of fills instead of pixel by pixel.
-// Against one pixel per thread with coverage in the record loop: 4.4 G against
+// Against one pixel per thread with coverage in the record loop: 4.7 G against
 // 8.5 G warp instructions on the 2048x2048 / 6,000-path frame, 6.1 against
 // 10.1 ms; 4096x4096 / 50,000 paths 128 against 207 ms, 1283x717 / 2,500 paths
 // 1.12 against 1.99 ms, 640x360 / 240 fills 0.26 against 0.29 ms.
