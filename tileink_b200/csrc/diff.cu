@@ -350,9 +350,7 @@ __global__ void __launch_bounds__(kDiffThreads)
     S.g[tid] = g;
     float(*const tc)[kDiffThreads] = reinterpret_cast<float(*)[kDiffThreads]>(S.c.rows);
     const uint32_t n_chunks = uint32_t((rec.ptcl_end - rec.ptcl_start + kDiffChunk - 1) / kDiffChunk);
-    // The tile's slots: tiles' records follow each other in tile order, so that with
-    // one slot more per tile for the rounding no two tiles share one.
-    float* const kept = scratch + (rec.ptcl_start / kDiffChunk + tile) * kDiffThreads + tid;
+    float* const kept = scratch + diff_scratch_at(rec.ptcl_start, tile) + tid;
     uint32_t m = 0;
     auto replay = [&](uint32_t chunk, float P) {
         const uint64_t r0 = rec.ptcl_start + uint64_t(chunk) * kDiffChunk;

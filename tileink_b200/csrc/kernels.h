@@ -323,10 +323,15 @@ void launch_stroke_emit(const StrokeView& v, const uint32_t* line_total, tk_path
 
 // Differentiable rendering (diff.cu): float forward and adjoint.
 constexpr uint32_t kDiffChunk = 16;  // records of a tile walked at a time
-// launch_diff_fine_bwd's scratch, in floats.
-constexpr uint64_t diff_scratch_len(uint64_t ptcl_used, uint64_t tiles) {
-    return (ptcl_used / kDiffChunk + tiles + 1u) * TK_TILE_SIZE * TK_TILE_SIZE;
+// launch_diff_fine_bwd's scratch: a float per pixel of each chunk. The first float of
+// the tile whose records start at ptcl_start (in 64 bits: beyond 2^24 chunks, 268 M
+// records, its number needs them). Tiles' records follow each other in tile order, so
+// that with one slot more per tile for the rounding no two tiles share one.
+__host__ __device__ constexpr uint64_t diff_scratch_at(uint64_t ptcl_start, uint64_t tile) {
+    return (ptcl_start / kDiffChunk + tile) * (TK_TILE_SIZE * TK_TILE_SIZE);
 }
+// Its length, in floats.
+constexpr uint64_t diff_scratch_len(uint64_t ptcl_used, uint64_t tiles) { return diff_scratch_at(ptcl_used, tiles + 1u); }
 void launch_diff_fine_fwd(const SceneView& s, const PassView& p, const float4* colp, float4* layer, cudaStream_t st);
 void launch_diff_blur(const float4* in, float4* out, const float* w, int32_t r, uint32_t width, uint32_t height,
                       int32_t axis, cudaStream_t st);
