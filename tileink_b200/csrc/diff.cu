@@ -41,7 +41,7 @@ constexpr uint32_t kDiffRows = 32;  // segments whose row parts are staged at a 
 struct DiffChunk {
     float4 colp[kDiffChunk];  // zero: no FILL record
     float base[kDiffChunk];   // the backdrop
-    uint32_t color[kDiffChunk];
+    uint32_t color[kDiffChunk];  // TK_INVALID_INDEX: no FILL record
     uint32_t end[kDiffChunk];     // inclusive prefix of the segment counts
     uint32_t offset[kDiffChunk];  // segment index of the chunk's j-th segment: offset + j
     float4 rows[kDiffRows][TK_TILE_SIZE];  // edge, dy, xmin, xmax of a segment in a pixel row
@@ -74,7 +74,7 @@ __device__ uint32_t stage_records(DiffChunk& S, const tk_ptcl_record* __restrict
         if (lane < kDiffChunk) {
             S.colp[lane] = fill ? colp[q.color] : make_float4(0.f, 0.f, 0.f, 0.f);
             S.base[lane] = fill ? float(q.backdrop) : 0.0f;
-            S.color[lane] = q.color;
+            S.color[lane] = fill ? q.color : TK_INVALID_INDEX;
             S.end[lane] = end;
             S.offset[lane] = q.segment_start - (end - n);
         }
@@ -399,8 +399,10 @@ __global__ void __launch_bounds__(kDiffThreads)
                     v[4] = fmaf(-t, S.P[r][i], v[4]);
                 }
                 const float s = warp_sum5(v, lane);
-                if (s != 0.0f && !(lane & 3u) && lane != 12u && lane < 24u)
-                    atomicAdd(color_acc + uint64_t(S.c.color[r]) * 5u + (lane >> 2) - (lane > 12u ? 1u : 0u), s);
+                const uint32_t color = S.c.color[r];
+                // (a record that is no FILL sums zeros, or NaN where g is not finite)
+                if (s != 0.0f && color != TK_INVALID_INDEX && !(lane & 3u) && lane != 12u && lane < 24u)
+                    atomicAdd(color_acc + uint64_t(color) * 5u + (lane >> 2) - (lane > 12u ? 1u : 0u), s);
             }
             if (!r0) break;
         }
