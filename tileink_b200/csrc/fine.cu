@@ -785,15 +785,11 @@ void launch_fine(const SceneView& s, const PassView& p, uint32_t* target, cudaSt
     // (4096^2, 50,000 paths: 207 -> 128 ms; 2048^2, 12,500 shapes: 1.62 here,
     // 1.65 there; 1280x800 glyph runs: 0.32 here, 0.49 ms there).
     if (!s.text && !s.sdf_words) return launch_fine_paths(s, p, target, T, st);
-    static bool configured = false;
-    if (!configured) {
-        for (auto k : {k_fine<1u, false>, k_fine<2u, false>, k_fine<0u, true>, k_fine<1u, true>, k_fine<2u, true>})
-            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(FineSmem)));
-        configured = true;
-    }
     if (s.sdf_ext) k_star_table<<<1, 32, 0, st>>>();
     auto kernel = s.text ? (!s.sdf_words ? k_fine<0u, true> : (s.sdf_ext ? k_fine<2u, true> : k_fine<1u, true>))
                          : (s.sdf_ext ? k_fine<2u, false> : k_fine<1u, false>);
+    // (an attribute of the device that the call is for)
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(FineSmem)));
     const GlyphView glyphs{p.glyph_list, s.glyphs, s.glyph_images, s.glyph_texels};
     kernel<<<T, kFineThreads, sizeof(FineSmem), st>>>(p.tiles, p.ptcl, s.segments, s.paints, s.brush, s.brush_words,
                                                       s.texels, s.draws, s.sdf, s.segment_capacity, target, s.width, s.height,

@@ -666,8 +666,7 @@ __device__ __noinline__ uint32_t rare_record(uint32_t* error, uint32_t tag, uint
 }
 
 __global__ void __launch_bounds__(kThreads, 7) k_fine_paths(const FineArgs a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    FineSmem& S = *reinterpret_cast<FineSmem*>(smem_raw);
+    __shared__ FineSmem S;
     const uint32_t tile = a.tile_list ? a.tile_list[blockIdx.x] : blockIdx.x;
     const tk_tile_record rec = a.tiles[tile];
     if (rec.ptcl_start >= rec.ptcl_end) return;
@@ -883,12 +882,7 @@ __global__ void __launch_bounds__(kThreads, 7) k_fine_paths(const FineArgs a) {
 }  // namespace
 
 void launch_fine_paths(const SceneView& s, const PassView& p, uint32_t* target, uint32_t tiles, cudaStream_t st) {
-    static bool configured = false;
-    if (!configured) {
-        cudaFuncSetAttribute(k_fine_paths, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(FineSmem)));
-        configured = true;
-    }
-    k_fine_paths<<<tiles, kThreads, sizeof(FineSmem), st>>>(
+    k_fine_paths<<<tiles, kThreads, 0, st>>>(
         FineArgs{p.tiles, p.ptcl, s.segments, s.paints, s.brush, s.brush_words, s.segment_capacity, target, s.width,
                  s.height, s.tw, s.error, p.scenes, p.tile_scene, p.tile_list, make_float2(-0.0f, -0.0f)});
 }

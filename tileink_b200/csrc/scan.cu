@@ -378,7 +378,7 @@ constexpr int kEmitThreads = 256;
 constexpr uint32_t kEmitWarps = kEmitThreads / 32;
 constexpr uint32_t kEmitPairs = 128;    // pairs of a group whose slots are held at a time
 constexpr uint32_t kEmitLong = 256;     // lines from which a whole CTA takes a path
-constexpr uint32_t kEmitWindow = 5632;  // cursors kept in shared memory (4 CTAs an SM)
+constexpr uint32_t kEmitWindow = 5600;  // cursors kept in shared memory: what the 48 KB that need no opt-in leave
 
 struct EmitGroups {
     Scan scan[kEmitWarps][32];
@@ -390,6 +390,7 @@ struct EmitSmem : EmitGroups {
     uint32_t ticket;
     uint32_t cursor[kEmitWindow];
 };
+static_assert(sizeof(EmitSmem) <= 48u * 1024u, "static shared memory, on every device alike");
 
 // Scan geometry of a path's lines g .. g + 31 in sc / first; the number of
 // their (line, step) pairs.
@@ -463,9 +464,8 @@ __global__ void __launch_bounds__(kEmitThreads, 4)
     k_scan_emit(const tk_line* __restrict__ lines, const tk_path_record* __restrict__ paths, uint32_t path_count,
                 uint32_t* cursors, SegmentRec* segments, uint64_t capacity, uint32_t* error, uint32_t* seg_line,
                 const uint32_t* __restrict__ order, uint32_t* ticket) {
-    extern __shared__ __align__(16) unsigned char emit_raw[];
     using Smem = std::conditional_t<LONG, EmitSmem, EmitGroups>;
-    Smem& S = *reinterpret_cast<Smem*>(emit_raw);
+    __shared__ Smem S;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t lt_mask = (1u << lane) - 1u;
     Scan* sc = S.scan[warp];
@@ -647,15 +647,9 @@ constexpr uint32_t kEmitFewPaths = 4u * 148u * 32u;
 
 template <bool LONG>
 void launch_emit_as(const SceneView& s, const uint32_t* order, uint32_t n, unsigned grid, cudaStream_t st) {
-    constexpr size_t bytes = LONG ? sizeof(EmitSmem) : sizeof(EmitGroups);
-    static bool configured = false;
-    if (!configured) {
-        cudaFuncSetAttribute(k_scan_emit<LONG>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
-        configured = true;
-    }
     cudaMemsetAsync(s.emit_ticket, 0, sizeof(uint32_t), st);
-    k_scan_emit<LONG><<<grid, kEmitThreads, bytes, st>>>(s.lines, s.paths, n, s.cursors, s.segments, s.segment_capacity,
-                                                         s.error, s.seg_line, order, s.emit_ticket);
+    k_scan_emit<LONG><<<grid, kEmitThreads, 0, st>>>(s.lines, s.paths, n, s.cursors, s.segments, s.segment_capacity,
+                                                     s.error, s.seg_line, order, s.emit_ticket);
 }
 
 void launch_emit(const SceneView& s, const uint32_t* order, uint32_t n, cudaStream_t st) {
