@@ -216,6 +216,7 @@ struct tk_ctx {
     bool rendered = false;
     // paths by decreasing line count: the order scan_emit's warps take them
     DBuf<uint32_t> emit_order;
+    uint32_t longest_path = 0;  // lines
     // line index per emitted segment (differentiable mode only)
     DBuf<uint32_t> seg_line;
     bool want_seg_line = false;
@@ -682,6 +683,8 @@ tk::SceneView view(tk_ctx* c) {
     s.infos = c->infos.ptr;
     s.emit_order = c->emit_order.ptr;
     s.emit_ticket = c->misc.ptr + 4;
+    s.longest_path = c->longest_path;
+    s.path_segments = c->bumps.ptr;
     return s;
 }
 
@@ -748,6 +751,7 @@ void upload_emit_order(tk_ctx* c) {
         for (uint32_t i = 0; i < n; ++i) tmp[count[(key[order[i]] >> shift) & 0xFFFFu]++] = order[i];
         order.swap(tmp);
     }
+    c->longest_path = most;
     upload(c->emit_order, order.data(), order.size(), c->stream);
 }
 
@@ -1047,7 +1051,9 @@ void scan_phase_partial(tk_ctx* c) {
     s.segment_capacity = device_plan ? c->segment_needed - 1 : c->host_segment_capacity;
     {
         StageMark m(c, 3);
-        tk::launch_scan_emit_paths(s, c->rescan_list.ptr, n, st);
+        uint64_t lines = 0;
+        for (uint32_t p : c->rescan) lines += c->h_paths[p].line_count;
+        tk::launch_scan_emit_paths(s, c->rescan_list.ptr, n, lines, c->h_paths[c->rescan[0]].line_count, st);
     }
     c->last_scan_paths = n;
     c->rescan.clear();

@@ -112,6 +112,8 @@ struct SceneView {
     DrawInfo* infos;             // per draw (launch_draw_table)
     const uint32_t* emit_order;  // paths by decreasing line count (optional)
     uint32_t* emit_ticket;       // path queue of scan_emit
+    uint32_t longest_path;       // the most lines of one path
+    const uint32_t* path_segments;  // segments per path (launch_path_totals; optional)
 };
 
 void launch_scan_count(const SceneView& s, cudaStream_t st);
@@ -129,7 +131,8 @@ void launch_scan_emit(const SceneView& s, cudaStream_t st);
 // clear their backdrop and count slices and count their lines; emit their
 // segments. Their pool scan runs through launch_pool_scan with their items.
 void launch_scan_count_paths(const SceneView& s, const uint32_t* list, uint32_t n, cudaStream_t st);
-void launch_scan_emit_paths(const SceneView& s, const uint32_t* list, uint32_t n, cudaStream_t st);
+void launch_scan_emit_paths(const SceneView& s, const uint32_t* list, uint32_t n, uint64_t lines, uint32_t longest,
+                            cudaStream_t st);
 // *changed = 1 when a listed path's segment total (bumps, from
 // launch_path_totals) differs from its planned segment_capacity.
 void launch_check_path_totals(const SceneView& s, const uint32_t* bumps, const uint32_t* list, uint32_t n,

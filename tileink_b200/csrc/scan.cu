@@ -392,14 +392,14 @@ struct EmitSmem : EmitGroups {
 };
 static_assert(sizeof(EmitSmem) <= 48u * 1024u, "static shared memory, on every device alike");
 
-// Scan geometry of a path's lines g .. g + 31 in sc / first; the number of
+// Scan geometry of a path's lines g .. g + size - 1 in sc / first; the number of
 // their (line, step) pairs.
 __device__ __forceinline__ uint32_t emit_group(const tk_line* __restrict__ lines, const tk_path_record& p, uint32_t pid,
-                                               uint32_t g, Scan* sc, uint32_t* first, uint32_t* error) {
+                                               uint32_t g, uint32_t size, Scan* sc, uint32_t* first, uint32_t* error) {
     const uint32_t lane = threadIdx.x & 31u, l = g + lane;
     Scan s;
     bool ok = false;
-    if (l < p.line_count) {
+    if (lane < size && l < p.line_count) {
         tk_line line = load_line(lines, uint64_t(p.line_start) + l);
         if (line.path_id != pid) atomicOr(error, ERR_LINE_PATH_MISMATCH);
         else ok = scan_geometry(line, p, s);
@@ -463,7 +463,7 @@ template <bool LONG>
 __global__ void __launch_bounds__(kEmitThreads, 4)
     k_scan_emit(const tk_line* __restrict__ lines, const tk_path_record* __restrict__ paths, uint32_t path_count,
                 uint32_t* cursors, SegmentRec* segments, uint64_t capacity, uint32_t* error, uint32_t* seg_line,
-                const uint32_t* __restrict__ order, uint32_t* ticket) {
+                const uint32_t* __restrict__ order, uint32_t* ticket, const uint32_t* __restrict__ path_segments) {
     using Smem = std::conditional_t<LONG, EmitSmem, EmitGroups>;
     __shared__ Smem S;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -489,10 +489,16 @@ __global__ void __launch_bounds__(kEmitThreads, 4)
             uint32_t* const cur = window ? S.cursor : cursors + p.data_offset;
             uint32_t* const slots = S.slot[warp];
             uint8_t* const owner = S.line[warp];
-            const uint32_t rounds = (p.line_count + kEmitThreads - 1u) / kEmitThreads;
+            // Lines that jump over many tiles: fewer per group, so that its pairs are held at once
+            // and the turn is not kept while the rest are computed (40 paths of 300 lines across
+            // 1000x1000: 0.54 ms by a warp each, 0.59 in groups of 32 lines, 0.23 in groups of 2).
+            uint32_t size = 32u;
+            const uint64_t pairs = path_segments ? __ldg(path_segments + pid) : 0u;
+            while (size > 1u && pairs * size > uint64_t(kEmitPairs) * p.line_count) size >>= 1;
+            const uint32_t rounds = (p.line_count + size * kEmitWarps - 1u) / (size * kEmitWarps);
             for (uint32_t it = 0; it < rounds; ++it) {
-                const uint32_t g = (it * kEmitWarps + warp) * 32u;
-                const uint32_t total = g < p.line_count ? emit_group(lines, p, pid, g, sc, first, error) : 0u;
+                const uint32_t g = (it * kEmitWarps + warp) * size;
+                const uint32_t total = g < p.line_count ? emit_group(lines, p, pid, g, size, sc, first, error) : 0u;
                 bool turn = it == 0u && warp == 0u;
                 // pairs b0 .. b0 + kEmitPairs - 1: their tiles, their slots in turn, their
                 // segments; the turn passes with the last of them
@@ -552,7 +558,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4)
         const uint32_t pid = order ? __ldg(order + k) : k;
         const tk_path_record p = load_path(paths, pid);
         for (uint32_t g = 0; g < p.line_count; g += 32u) {
-            const uint32_t total = emit_group(lines, p, pid, g, sc, first, error);
+            const uint32_t total = emit_group(lines, p, pid, g, 32u, sc, first, error);
             for (uint32_t base = 0; base < total; base += 32u) {
                 const uint32_t j = base + lane;
                 bool emitting = false;
@@ -639,28 +645,39 @@ void launch_scan_count_paths(const SceneView& s, const uint32_t* list, uint32_t 
 
 namespace {
 
-// Whole CTAs take the long paths while there are few paths for the GPU's 4,736
-// resident warps (6,000 paths: 0.77 against 1.57 ms); beyond that single warps
-// keep it busy (50,000 paths: 7.7 against 10.5 ms; 35,000 paths of a batch: 1.1
-// against 1.5 ms).
-constexpr uint32_t kEmitFewPaths = 4u * 148u * 32u;
+// With a warp per path the kernel lasts as long as the longest path, or the mean load of
+// the GPU's resident warps; with whole CTAs for the long ones the latter, over the share of
+// the CTA's warps that a mean path keeps busy (its lines in whole rounds of kEmitThreads).
+// The CTAs pay from 1.5 times that on: ms with a warp per path and with CTAs (mixed scenes of
+// 2,700 lines a path at 2048x2048, others with lines of 8 px at 1024x1024):
+//   3,000 paths 1.28, 0.40; 9,000: 1.63, 1.12; 12,000 (longest 1.6 times the mean load):
+//   1.68, 1.48; 18,900 (1.0 times): 1.90, 1.88
+//   300 lines each: 600 paths 0.040, 0.027; 2,500 (1.9 times, but 300 of 512): 0.051, 0.059;
+//   5,000: 0.083, 0.106; 9,000 fills of 1,360 lines (1.0 times): 0.63, 0.78
+constexpr uint64_t kEmitResident = 4u * 148u * kEmitWarps;
 
 template <bool LONG>
 void launch_emit_as(const SceneView& s, const uint32_t* order, uint32_t n, unsigned grid, cudaStream_t st) {
     cudaMemsetAsync(s.emit_ticket, 0, sizeof(uint32_t), st);
     k_scan_emit<LONG><<<grid, kEmitThreads, 0, st>>>(s.lines, s.paths, n, s.cursors, s.segments, s.segment_capacity,
-                                                     s.error, s.seg_line, order, s.emit_ticket);
+                                                     s.error, s.seg_line, order, s.emit_ticket, s.path_segments);
 }
 
-void launch_emit(const SceneView& s, const uint32_t* order, uint32_t n, cudaStream_t st) {
-    if (n < kEmitFewPaths) launch_emit_as<true>(s, order, n, grid_for(n, 1, 148 * 4), st);
-    else launch_emit_as<false>(s, order, n, grid_for(uint64_t(n) * 32, kEmitThreads, 148 * 8), st);
+// `lines`: of the n paths together, `longest` of one.
+void launch_emit(const SceneView& s, const uint32_t* order, uint32_t n, uint64_t lines, uint32_t longest,
+                 cudaStream_t st) {
+    const uint64_t mean = (lines / n + kEmitThreads - 1u) / kEmitThreads * kEmitThreads;
+    if (longest >= kEmitLong && 2u * kEmitResident * longest >= 3u * n * mean)
+        launch_emit_as<true>(s, order, n, grid_for(n, 1, 148 * 4), st);
+    else
+        launch_emit_as<false>(s, order, n, grid_for(uint64_t(n) * 32, kEmitThreads, 148 * 8), st);
 }
 
 }  // namespace
 
-void launch_scan_emit_paths(const SceneView& s, const uint32_t* list, uint32_t n, cudaStream_t st) {
-    if (n) launch_emit(s, list, n, st);
+void launch_scan_emit_paths(const SceneView& s, const uint32_t* list, uint32_t n, uint64_t lines, uint32_t longest,
+                            cudaStream_t st) {
+    if (n) launch_emit(s, list, n, lines, longest, st);
 }
 
 void launch_check_path_totals(const SceneView& s, const uint32_t* bumps, const uint32_t* list, uint32_t n,
@@ -670,7 +687,7 @@ void launch_check_path_totals(const SceneView& s, const uint32_t* bumps, const u
 }
 
 void launch_scan_emit(const SceneView& s, cudaStream_t st) {
-    if (s.path_count) launch_emit(s, s.emit_order, s.path_count, st);
+    if (s.path_count) launch_emit(s, s.emit_order, s.path_count, s.line_count, s.longest_path, st);
 }
 
 }  // namespace tk
