@@ -1323,16 +1323,16 @@ void flatten_on_device(tk_ctx* c, const tk_scene_desc& d, const tk_flatten_desc&
     upload(c, sels, fl.stroke_elements, nse, st);
     upload(polys, fl.polylines, npl, st);
     upload(strokes, fl.strokes, ns, st);
-    offsets.reserve(n);
+    offsets.reserve(2 * n);  // and the list of the longer elements
     sums.reserve(tk::flatten_block_sums(n));
     soff.reserve(nse);
     ssums.reserve(tk::flatten_block_sums(std::max<uint64_t>(nse, npl)));
     poly_n.reserve(npl);
     line_off.reserve(npl);
-    // words: [0] fill lines [1] error [2] stroke points [3] stroke lines
-    words.reserve(4);
+    // words: [0] fill lines [1] error [2] stroke points [3] stroke lines [4] longer elements
+    words.reserve(5);
     wide.reserve(2);  // exact sums: [0] stroke points [1] stroke lines
-    TK_CUDA(cudaMemsetAsync(words.ptr, 0, 4 * sizeof(uint32_t), st));
+    TK_CUDA(cudaMemsetAsync(words.ptr, 0, 5 * sizeof(uint32_t), st));
     TK_CUDA(cudaMemsetAsync(wide.ptr, 0, 2 * sizeof(unsigned long long), st));
     tk::launch_flatten_count(els.ptr, n, offsets.ptr, sums.ptr, words.ptr, words.ptr + 1, st);
     tk::launch_stroke_count(sels.ptr, nse, soff.ptr, ssums.ptr, words.ptr + 2, wide.ptr, words.ptr + 1, st);
@@ -1363,7 +1363,7 @@ void flatten_on_device(tk_ctx* c, const tk_scene_desc& d, const tk_flatten_desc&
     c->lines.reserve(total);
     copy_in(c, c->lines.ptr, d.lines, host_lines * sizeof(tk_line), st);
     tk::launch_flatten_emit(els.ptr, n, offsets.ptr, words.ptr, c->paths.ptr, d.path_count, path_els.ptr, c->lines.ptr,
-                            host_lines, host_lines + fill_lines, words.ptr + 1, st);
+                            host_lines, host_lines + fill_lines, offsets.ptr + n, words.ptr + 4, words.ptr + 1, st);
     tk::launch_stroke_emit(sv, words.ptr + 3, c->paths.ptr, c->lines.ptr, host_lines + fill_lines, total, st);
     TK_CUDA(cudaGetLastError());
     uint32_t err = 0;

@@ -285,11 +285,13 @@ int32_t launch_blur_downsampled(uint32_t* surface, uint32_t* low, uint32_t* temp
 
 // Device flattening (flatten.cu): per-element line counts, exclusive offsets
 // in `counts` and the total; then path line ranges and the lines themselves.
+// `longs` has room for n elements, and *long_count is 0.
 void launch_flatten_count(const tk_flatten_el* els, uint64_t n, uint32_t* counts, uint32_t* block_sums,
                           uint32_t* total, uint32_t* error, cudaStream_t st);
 void launch_flatten_emit(const tk_flatten_el* els, uint64_t n, const uint32_t* offsets, const uint32_t* total,
                          tk_path_record* paths, uint32_t path_count, const uint32_t* path_els, tk_line* lines,
-                         uint64_t line_base, uint64_t line_end, uint32_t* error, cudaStream_t st);
+                         uint64_t line_base, uint64_t line_end, uint32_t* longs, uint32_t* long_count, uint32_t* error,
+                         cudaStream_t st);
 size_t flatten_block_sums(uint64_t n);
 // Exclusive scan of n u32 values in place (1024 per block; block totals in
 // block_sums, flatten_block_sums(n) words); `total` receives the sum.
