@@ -1,7 +1,7 @@
 // Separable Gaussian blur and surface composite.
 //
 // Shared route (radius <= 16, filter/blur_shared.hlsl:15-74): a CTA stages a
-// 32x32 pixel tile plus the +-radius halo along the blurred axis in shared
+// 32x32 pixel tile (32x8 in small regions) plus the +-radius halo along the blurred axis in shared
 // memory; every pixel accumulates its taps in the reference's order with
 // fused multiply-adds. The Gaussian weight recurrence
 // (w_{d+1} = w_d * ratio, ratio *= decay) and the normalising sum are the
@@ -23,6 +23,8 @@ using namespace tkd;
 
 constexpr int kTile = 32, kOut = 4;  // a thread has kOut pixels along the blurred axis
 constexpr int kPitch = kTile + 1;
+constexpr int kRows = 8;              // of a small region's tile
+constexpr uint32_t kFewTiles = 100;   // fewer 32x32 tiles than this, two thirds of the SMs: a small region
 constexpr int kMaxR = int(TK_SHARED_BLUR_MAX_RADIUS);
 
 constexpr int kMaxWide = 48;
@@ -137,6 +139,39 @@ __global__ void __launch_bounds__(kTile * kTile / kOut)
                 dst[uint64_t(y) * width + x] = s[lane][warp + k * (kTile / kOut)];
         }
     }
+}
+
+// The same with a pixel per thread on 32x8 tiles, for regions of fewer than kFewTiles
+// 32x32 tiles: what counts there is how soon a thread is done. Both passes, us, with the
+// kernel above and this one, radius 12: 4 tiles 20.9, 16.4; 81 tiles 23.0, 20.8; 144 tiles
+// 23.0, 23.0; radius 16: 81 tiles 23.0, 23.1; 100 tiles 23.0, 26.8.
+template <int AXIS>
+__global__ void __launch_bounds__(kTile * kRows)
+    k_blur_small(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, uint32_t width, uint32_t height,
+                 uint4 region, int4 bounds, Weights wt) {
+    __shared__ uint32_t s[AXIS == 0 ? kRows * (kTile + 2 * kMaxR) : (kRows + 2 * kMaxR) * kTile];
+    const int r = wt.r, lx = threadIdx.x % kTile, ly = threadIdx.x / kTile;
+    const int ox = int(region.x) + int(blockIdx.x) * kTile, oy = int(region.y) + int(blockIdx.y) * kRows;
+    const int hx = AXIS == 0 ? r : 0, hy = AXIS == 0 ? 0 : r, sw = kTile + 2 * hx, sh = kRows + 2 * hy;
+    for (int cy = ly; cy < sh; cy += kRows)
+        for (int cx = lx; cx < sw; cx += kTile) {
+            const int x = ox - hx + cx, y = oy - hy + cy;
+            uint32_t v = 0u;
+            if (inside_b(x, y, bounds) && x >= 0 && y >= 0 && x < int(width) && y < int(height))
+                v = src[uint64_t(y) * width + x];
+            s[cy * sw + cx] = v;
+        }
+    __syncthreads();
+    const int x = ox + lx, y = oy + ly;
+    if (x >= int(region.x + region.z) || y >= int(region.y + region.w) || x >= int(width) || y >= int(height)) return;
+    const int at = (ly + hy) * sw + lx + hx, step = AXIS == 0 ? 1 : sw;
+    Texel acc = unpack(s[at]);
+    for (int d = 1; d <= r; ++d) {
+        const float w = wt.w[d];
+        acc_texel(acc, unpack(s[at + d * step]), w);
+        acc_texel(acc, unpack(s[at - d * step]), w);
+    }
+    dst[uint64_t(y) * width + x] = pack_average(make_float4(acc.rg.x, acc.rg.y, acc.ba.x, acc.ba.y), wt.inv_sum);
 }
 
 // filter/sample.hlsli:4-17 on an RGBA8 source (texel loads are k/255).
@@ -446,7 +481,12 @@ void launch_blur(const uint32_t* src, uint32_t* dst, const BlurParams& b, cudaSt
         ratio = ratio * decay;
     }
     wt.inv_sum = 1.0f / sum;
-    dim3 grid((rw + kTile - 1) / kTile, (rh + kTile - 1) / kTile);
+    const dim3 grid((rw + kTile - 1) / kTile, (rh + kTile - 1) / kTile), small(grid.x, (rh + kRows - 1) / kRows);
+    if (grid.x * grid.y < kFewTiles) {
+        if (b.axis == 0) k_blur_small<0><<<small, kTile * kRows, 0, st>>>(src, dst, b.width, b.height, region, bounds, wt);
+        else k_blur_small<1><<<small, kTile * kRows, 0, st>>>(src, dst, b.width, b.height, region, bounds, wt);
+        return;
+    }
     if (b.axis == 0)
         k_blur_shared<0><<<grid, kTile * kTile / kOut, 0, st>>>(src, dst, b.width, b.height, region, bounds, wt);
     else
