@@ -29,8 +29,8 @@
 //     pixels, in zero-filled blocks of four, one product per lane;
 //   - the segments that touch the tile's left edge: only they add to `base`
 //     (the row edges of the others are +-0, which leave the sum unchanged).
-// A lane then takes half a row of one fill and accumulates base, `running` and
-// `partial` of its 8 pixels in segment order over the row's entries exactly as
+// A lane then takes half a row of one fill (a quarter where the chunk has one or two
+// fills) and accumulates base, `running` and `partial` of its pixels in segment order over the row's entries exactly as
 // fill_alpha_at (shared/coverage.hlsli:34-51) does, so the f32 sums are the
 // reference's; the rows are taken in order of their number of entries (2 to 3
 // on average, 6 at the longest of 32 rows), so that a warp's lanes end together.
@@ -167,14 +167,100 @@ __device__ __forceinline__ bool stage_fits(uint32_t pre) {
     return (pre & 0xFFFu) <= kItems && ((pre >> 12) & 0xFFFu) < kBlocks;
 }
 
+// The coverage of the fills' rows, 16 / PARTS pixels per lane. Sliced: those of a single
+// record's slice, thread PARTS r + h part h of row r; its sums start from `carry` when carried
+// and end there when it is not the last slice (partly).
+// Quarter rows spend a quarter more instructions a row than half rows, but one or two
+// fills' half rows leave two or three of the four warps idle: with quarters there,
+// 2048x2048 / 6,000 paths 6.1 -> 5.8 ms, 640x360 / 240 fills 0.26 -> 0.245, 96x80 / 8 paths
+// of 5,000 lines (slices) 2.4 -> 2.1, and 1.78 with the largest slices that fit.
+template <uint32_t PARTS>
+__device__ __forceinline__ void cover_rows(FineSmem& S, uint32_t fills, uint32_t total, uint32_t first, bool sliced,
+                                           bool carried, bool partly, float2 nz, float2 (&carry)[5]) {
+    constexpr uint32_t kPairs = TK_TILE_SIZE / PARTS / 2u;  // pixel pairs of a lane
+    const uint32_t tid = threadIdx.x;
+    const uint32_t rows0 = __shfl_sync(0xffffffffu, first, (tid / PARTS) & 15u);  // the first entry of row tid / PARTS, when sliced
+    const unsigned char* prod = reinterpret_cast<const unsigned char*>(S.prod);
+#pragma unroll 1
+    for (uint32_t ci = tid; ci < fills * TK_TILE_SIZE * PARTS; ci += kThreads) {
+        const uint32_t part = ci % PARTS;
+        uint32_t w = S.rows[ci / PARTS];
+        if (PARTS == 4u && sliced) {
+            const unsigned char* at = reinterpret_cast<const unsigned char*>(S.pos) + ci / PARTS;
+            w = rows0 | (uint32_t(at[total * TK_TILE_SIZE] - at[0]) << 12) | ((ci / PARTS) << 20);
+        }
+        const uint32_t f = w >> 24, r = (w >> 20) & 15u;
+        const uint4 h = S.hdr[S.cover[f]];
+        float base = PARTS == 4u && carried ? carry[4].x : __uint_as_float(h.z);
+#pragma unroll 1
+        for (uint32_t e = (h.y >> 16) & 255u, e1 = h.y >> 24; e < e1; ++e)
+            base += S.edge[e].y * clampf(float(r) - S.edge[e].x + 1.0f, 0.0f, 1.0f);
+        float2 running[kPairs], partial[kPairs];
+#pragma unroll
+        for (uint32_t q = 0; q < kPairs; ++q) {
+            running[q] = partial[q] = make_float2(0.0f, 0.0f);
+            if (PARTS == 4u && carried) {
+                running[q] = carry[q];
+                partial[q] = carry[q + 2u];
+            }
+        }
+        const float x4 = 2.0f + float(part) * (64.0f / PARTS);
+        const float4* e = S.ent + (w & 0xFFFu);
+        const float4* const e1 = e + ((w >> 12) & 255u);
+#pragma unroll 1
+        for (; e < e1; ++e) {
+            const float4 c = *e;
+            const uint32_t o = __float_as_uint(part >= PARTS / 2u ? c.w : c.z);
+            const float t = c.y + x4;
+#pragma unroll
+            for (uint32_t q = 0; q < kPairs; ++q) {
+                // 1 for pixels x >= phi, else 0: clamp(4 (x - phi) + 2, 0, 1)
+                const float2 m = make_float2(__saturatef(t + 8.0f * float(q)), __saturatef(t + (8.0f * float(q) + 4.0f)));
+                running[q] = __ffma2_rn(both(c.x), m, running[q]);  // + dy or + 0
+            }
+#pragma unroll
+            for (uint32_t q = 0; q < kPairs; q += 2u) {
+                const uint32_t at = PARTS == 4u ? (part & 1u ? o >> 16 : o & 0xFFFFu) : (q ? o >> 16 : o & 0xFFFFu);
+                const float4 p = *reinterpret_cast<const float4*>(prod + at);
+                partial[q] = add2(partial[q], make_float2(p.x, p.y));
+                partial[q + 1u] = add2(partial[q + 1u], make_float2(p.z, p.w));
+            }
+        }
+        if (PARTS == 4u && partly) {
+            carry[4].x = base;
+#pragma unroll
+            for (uint32_t q = 0; q < 2u; ++q) {
+                carry[q] = running[q];
+                carry[q + 2u] = partial[q];
+            }
+            continue;
+        }
+        const bool even_odd = (h.x & kHdrEvenOdd) != 0u;
+#pragma unroll
+        for (uint32_t g = 0; g < kPairs / 2u; ++g) {
+            float2 v[2];
+            v[0] = add2(add2(both(base), running[2 * g]), partial[2 * g]);
+            v[1] = add2(add2(both(base), running[2 * g + 1]), partial[2 * g + 1]);
+            uint32_t word;
+            if (even_odd && fabsf(base) > 1.0e6f) {  // windings that coverage_bytes does not fold
+                word = coverage_to_alpha(v[0].x, 1u) | (coverage_to_alpha(v[0].y, 1u) << 8) |
+                       (coverage_to_alpha(v[1].x, 1u) << 16) | (coverage_to_alpha(v[1].y, 1u) << 24);
+            } else {
+                word = coverage_bytes(v, even_odd ? 2.0f : 0.0f, nz);
+            }
+            reinterpret_cast<uint32_t*>(S.alpha)[((f * TK_TILE_SIZE + r) * PARTS + part) * (kPairs / 2u) + g] = word;
+        }
+    }
+}
+
 // Stages the crossing entries and products of the chunk's first n records,
 // whose `total` segments are staged, and the coverage alphas of their fills;
 // `n` and `total` become the records and segments that the shared arrays hold.
 // A single record (n == 1) is taken in as many slices of its segments as it
-// needs: `before` are done already and `left` are not, and thread 2 r + h carries
-// the sums of half h of row r from slice to slice (its alphas count after the last).
+// needs: `before` are done already and `left` are not, and `carry` holds the sums from
+// slice to slice (cover_rows; its alphas count after the last).
 __device__ __forceinline__ void stage_coverage(FineSmem& S, uint32_t& n, uint32_t& total, uint32_t before,
-                                               uint32_t left, float2 nz, float2 (&carry)[9]) {
+                                               uint32_t left, float2 nz, float2 (&carry)[5]) {
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     // Prefixes over the segments: four words of four row counters (bytes), and
     // one of crossings, product blocks (what a segment can need: one per row and
@@ -212,8 +298,16 @@ __device__ __forceinline__ void stage_coverage(FineSmem& S, uint32_t& n, uint32_
             n = max(uint32_t(__popc(__ballot_sync(0xffffffffu, fit))), 1u);
             total = S.off[n];
         }
-        // one record: a slice whose crossings fit (a segment has at most 16)
-        while (n == 1u && total > 1u && !stage_fits(S.pre[total])) total >>= 1;
+        // one record: the largest slice whose crossings and blocks fit (one segment's do)
+        if (n == 1u && !stage_fits(S.pre[total])) {
+            uint32_t fit = 1u;
+            while (total - fit > 1u) {
+                const uint32_t mid = (fit + total) >> 1;
+                if (stage_fits(S.pre[mid])) fit = mid;
+                else total = mid;
+            }
+            total = fit;
+        }
         const uint32_t items = S.pre[total] & 0xFFFu;
         const uint32_t count = lane < TK_TILE_SIZE ? pos[total * TK_TILE_SIZE + lane] : 0u;
         first = warp_inclusive(count, lane) - count;  // the first entry of tile row `lane`
@@ -335,79 +429,13 @@ __device__ __forceinline__ void stage_coverage(FineSmem& S, uint32_t& n, uint32_
         __syncthreads();
     }
     __syncthreads();
-    // fill_alpha_at's coverage sums and coverage_to_alpha, half a fill's row per lane
+    // fill_alpha_at's coverage sums and coverage_to_alpha: half a fill's row per lane, or a
+    // quarter where there are too few fills for the CTA's threads
     const bool partly = n == 1u && total < (before != 0u ? left : S.off[1]), sliced = n == 1u && (partly || before != 0u);
-    const uint32_t rows0 = __shfl_sync(0xffffffffu, first, (lane >> 1) & 15u);  // the first entry of row tid / 2, for tid < 32
-    const unsigned char* prod = reinterpret_cast<const unsigned char*>(S.prod);
-#pragma unroll 1
-    for (uint32_t ci = tid; ci < fills * TK_TILE_SIZE * 2u; ci += kThreads) {
-        uint32_t w = S.rows[ci >> 1];
-        if (sliced) {
-            const unsigned char* at = reinterpret_cast<const unsigned char*>(S.pos) + (ci >> 1);
-            w = rows0 | (uint32_t(at[total * TK_TILE_SIZE] - at[0]) << 12) | ((ci >> 1) << 20);
-        }
-        const uint32_t f = w >> 24, r = (w >> 20) & 15u;
-        const bool right = (ci & 1u) != 0u;
-        const uint4 h = S.hdr[S.cover[f]];
-        const bool carried = sliced && before != 0u;
-        float base = carried ? carry[8].x : __uint_as_float(h.z);
-#pragma unroll 1
-        for (uint32_t e = (h.y >> 16) & 255u, e1 = h.y >> 24; e < e1; ++e)
-            base += S.edge[e].y * clampf(float(r) - S.edge[e].x + 1.0f, 0.0f, 1.0f);
-        float2 running[4], partial[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) running[q] = partial[q] = make_float2(0.0f, 0.0f);
-        if (carried)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                running[q] = carry[q];
-                partial[q] = carry[q + 4];
-            }
-        const float x4 = right ? 34.0f : 2.0f;
-        const float4* e = S.ent + (w & 0xFFFu);
-        const float4* const e1 = e + ((w >> 12) & 255u);
-#pragma unroll 1
-        for (; e < e1; ++e) {
-            const float4 c = *e;
-            const uint32_t o = __float_as_uint(right ? c.w : c.z);
-            const float t = c.y + x4;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                // 1 for pixels x >= phi, else 0: clamp(4 (x - phi) + 2, 0, 1)
-                const float2 m = make_float2(__saturatef(t + 8.0f * float(q)), __saturatef(t + (8.0f * float(q) + 4.0f)));
-                running[q] = __ffma2_rn(both(c.x), m, running[q]);  // + dy or + 0
-            }
-            const float4 p = *reinterpret_cast<const float4*>(prod + (o & 0xFFFFu));
-            const float4 u = *reinterpret_cast<const float4*>(prod + (o >> 16));
-            partial[0] = add2(partial[0], make_float2(p.x, p.y));
-            partial[1] = add2(partial[1], make_float2(p.z, p.w));
-            partial[2] = add2(partial[2], make_float2(u.x, u.y));
-            partial[3] = add2(partial[3], make_float2(u.z, u.w));
-        }
-        if (partly) {
-            carry[8].x = base;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                carry[q] = running[q];
-                carry[q + 4] = partial[q];
-            }
-            continue;
-        }
-        const bool even_odd = (h.x & kHdrEvenOdd) != 0u;
-        uint32_t words[2];
-#pragma unroll
-        for (int g = 0; g < 2; ++g) {
-            float2 v[2];
-            v[0] = add2(add2(both(base), running[2 * g]), partial[2 * g]);
-            v[1] = add2(add2(both(base), running[2 * g + 1]), partial[2 * g + 1]);
-            if (even_odd && fabsf(base) > 1.0e6f) {  // windings that coverage_bytes does not fold
-                words[g] = coverage_to_alpha(v[0].x, 1u) | (coverage_to_alpha(v[0].y, 1u) << 8) |
-                           (coverage_to_alpha(v[1].x, 1u) << 16) | (coverage_to_alpha(v[1].y, 1u) << 24);
-            } else {
-                words[g] = coverage_bytes(v, even_odd ? 2.0f : 0.0f, nz);
-            }
-        }
-        reinterpret_cast<uint2*>(S.alpha)[(f * TK_TILE_SIZE + r) * 2u + (ci & 1u)] = make_uint2(words[0], words[1]);
+    if (fills > 2u) {
+        cover_rows<2>(S, fills, total, first, false, false, false, nz, carry);
+    } else {
+        cover_rows<4>(S, fills, total, first, sliced, sliced && before != 0u, partly, nz, carry);
     }
     __syncthreads();
 }
@@ -664,7 +692,6 @@ __device__ __noinline__ uint32_t rare_record(uint32_t* error, uint32_t tag, uint
     }
     return gdepth;
 }
-
 __global__ void __launch_bounds__(kThreads, 7) k_fine_paths(const FineArgs a) {
     __shared__ FineSmem S;
     const uint32_t tile = a.tile_list ? a.tile_list[blockIdx.x] : blockIdx.x;
@@ -704,7 +731,7 @@ __global__ void __launch_bounds__(kThreads, 7) k_fine_paths(const FineArgs a) {
     uint32_t cdepth = 0u, gdepth = 0u;
     Group groups[kGroupDepth];
     uint32_t mode = TK_TILE_KIND_INTERPRETER;
-    float2 carry[9];
+    float2 carry[5];
 
     uint64_t r = rec.ptcl_start;
     const uint64_t end = rec.ptcl_end;
