@@ -1,12 +1,13 @@
 """Fine raster of path-only scenes: chunks of one, two and three fills (quarter and half
-rows per lane) and records taken in slices of every length, bit for bit against the
-oracle."""
+rows per lane), records taken in slices of every length, and the instances with and
+without opacity groups, bit for bit against the oracle."""
 import numpy as np
 import pytest
 
 import tileink_b200 as tk
+from tileink_b200 import NativeRenderer
 
-from test_gpu_fine_paths import STOPS, zigzag
+from test_gpu_fine_paths import STOPS, rect, zigzag
 from test_gpu_parity import compare_frame
 
 pytestmark = pytest.mark.gpu
@@ -46,3 +47,44 @@ def test_gpu_fine_slice_lengths(renderer, steep):
     c.push_path(p.close(), tk.Brush.solid(0.9, 0.2, 0.1, 0.8), fill_rule=tk.FILL_EVEN_ODD)
     c.push_path(zigzag(2.0, 14.0, 1.0, 15.0, 150), tk.Brush.solid(0.1, 0.3, 0.9, 0.6))
     compare_frame(renderer, c)
+
+
+def grouped(opacity, w, h):
+    rng = np.random.default_rng(5)
+    c = tk.Canvas(w, h)
+    c.set_clear_color(0xFFFFFFFF)
+    c.push_clip_layer(rect(3.5, 2.5, w - 4.2, h - 3.1))
+    c.push_path(rect(-1, -1, w + 1, h + 1), tk.Brush.solid(0.2, 0.4, 0.9, 1.0))  # a colour under a clip
+    for depth in (1, 2, 5):  # up to more groups than are kept as floats
+        for k in range(depth):
+            if opacity:
+                c.push_opacity_layer(star(rng, 9, w, h), 0.8 - 0.05 * k)
+            else:
+                c.push_clip_layer(star(rng, 9, w, h))
+        for _ in range(3):
+            c.push_path(star(rng, 12, w, h), tk.Brush.solid(*rng.uniform(0, 1, 3), 0.6))
+        for _ in range(depth):
+            c.pop_layer()
+    c.pop_layer()
+    c.push_path(star(rng, 20, w, h), tk.Brush.solid(0.9, 0.5, 0.1, 0.5))
+    return c
+
+
+@pytest.mark.parametrize("opacity", [False, True])
+def test_gpu_fine_group_instances(renderer, opacity):
+    compare_frame(renderer, grouped(opacity, 49, 35))
+
+
+@pytest.mark.parametrize("with_groups", [(), (2,), (0, 1, 2)])
+def test_gpu_fine_groups_in_a_batch(with_groups):
+    """A batch takes the instance with groups as soon as one of its scenes has them."""
+    scenes = [grouped(k in with_groups, 40 + 9 * k, 33) for k in range(3)]
+    r, one = NativeRenderer(0), NativeRenderer(0)
+    try:
+        r.batch_upload(scenes)
+        r.batch_render()
+        for got, scene in zip(r.batch_readback(), scenes):
+            assert np.array_equal(got, one.render_to_image(scene))
+    finally:
+        r.close()
+        one.close()

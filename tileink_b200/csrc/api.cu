@@ -178,6 +178,7 @@ struct tk_ctx {
     uint64_t sdf_words = 0, sdf_shadow_base = 0;  // SDF buffer: sdf_blob, then sdf_shadow_blob
     bool sdf_ext = false;                          // a candlestick, dash line, triangle or checkerboard
     bool text = false;                             // glyph outline fills or glyph runs
+    bool groups = false;                           // opacity layers
     uint32_t path_count = 0, draw_count = 0, layer_count = 0, order_count = 0;
     std::vector<tk_path_record> h_paths;
     std::vector<tk::ScanItem> h_items;
@@ -392,7 +393,7 @@ void validate_and_plan(tk_ctx* c, const tk_scene_desc& d) {
             invalid("glyph image " + std::to_string(k) + " outside the glyph texels");
     }
     bool sdf_ext = false;
-    bool text = false;
+    bool text = false, groups = false;
     // Draws: path fills/clips, and brush draws of the SDF kinds this library
     // renders (one complete record each, src/shared/gpu_sdf.rs:27-46).
     for (uint32_t i = 0; i < d.draw_count; ++i) {
@@ -457,6 +458,7 @@ void validate_and_plan(tk_ctx* c, const tk_scene_desc& d) {
         if (d.layers[i].tag == TK_LAYER_BLEND) invalid("blend layers are outside this path");
         if (d.layers[i].tag > TK_LAYER_BLEND) invalid("bad layer tag");
         if (d.layers[i].draw >= d.draw_count) invalid("layer draw out of range");
+        if (d.layers[i].tag == TK_LAYER_OPACITY) groups = true;
         const tk_draw_record& ld = d.draws[d.layers[i].draw];
         const bool sdf_clip = ld.sdf_offset != TK_INVALID_INDEX && ld.tag == TK_DRAW_CLIP;
         if (sdf_clip ? d.layers[i].tag != TK_LAYER_CLIP : ld.path_id == TK_INVALID_INDEX)
@@ -623,6 +625,7 @@ void validate_and_plan(tk_ctx* c, const tk_scene_desc& d) {
     c->sdf_ext = sdf_ext;
     c->glyph_run_count = d.glyph_run_count;
     c->text = text;
+    c->groups = groups;
     c->pool_len = pool;
     c->host_segment_capacity = seg_cap;
     c->h_paths.assign(d.paths, d.paths + d.path_count);
@@ -655,6 +658,7 @@ tk::SceneView view(tk_ctx* c) {
     s.sdf_shadow_base = c->sdf_shadow_base;
     s.sdf_ext = c->sdf_ext;
     s.text = c->text;
+    s.groups = c->groups;
     s.texels = c->texels.ptr;
     if (c->glyph_run_count) {
         s.glyph_runs = c->glyph_runs.ptr;
@@ -1409,7 +1413,7 @@ void do_batch_upload(tk_ctx* c, const tk_scene_desc* scenes, uint32_t n) {
     uint64_t pool = 0, segs = 0, list = 0, pixels = 0;
     uint32_t tiles = 0, bins = 0, batch_base = 0;
     bool ext = false;  // some scene has SDF records of an extended kind
-    bool text = false;  // some scene has glyph outline fills
+    bool text = false, groups = false;  // some scene has glyph outline fills, opacity layers
     for (uint32_t s = 0; s < n; ++s) {
         const tk_scene_desc& d = scenes[s];
         if (d.flags & TK_SCENE_SEGMENTS_FROM_DEVICE) invalid("batched scenes use host segment planning");
@@ -1418,6 +1422,7 @@ void do_batch_upload(tk_ctx* c, const tk_scene_desc* scenes, uint32_t n) {
         validate_and_plan(c, d);
         ext = ext || c->sdf_ext;
         text = text || c->text;
+        groups = groups || c->groups;
         uint32_t npass = 0;
         for (const Step& st : c->steps) {
             if (st.kind != STEP_PASS) invalid("scene " + std::to_string(s) + ": blur groups are not batched");
@@ -1531,6 +1536,7 @@ void do_batch_upload(tk_ctx* c, const tk_scene_desc* scenes, uint32_t n) {
     c->sdf_shadow_base = sdf.size();
     c->sdf_ext = ext;
     c->text = text;
+    c->groups = groups;
     sdf.insert(sdf.end(), shadow.begin(), shadow.end());
     c->sdf_words = sdf.size();
     c->pool_len = pool;
