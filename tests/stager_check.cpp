@@ -1,0 +1,51 @@
+// The upload ring on the CPU (tests/test_stager.py): stager_check MODE, 0 when it holds.
+#include <chrono>
+#include <cstdio>
+#include <ctime>
+#include <string>
+
+#include "stager.h"
+
+using tk::Stager;
+
+static std::vector<uint8_t> bytes(size_t n, uint32_t seed) {
+    std::vector<uint8_t> v(n);
+    uint32_t x = seed * 2654435761u + 1u;
+    for (size_t i = 0; i < n; ++i) {
+        x = x * 1664525u + 1013904223u;
+        v[i] = uint8_t(x >> 24);
+    }
+    return v;
+}
+
+static void rest(int ms) { std::this_thread::sleep_for(std::chrono::milliseconds(ms)); }
+
+// Uploads of the sizes from several threads through one ring, as the library makes them.
+static int data() {
+    auto ring = Stager::of(0);
+    std::atomic<int> wrong{0};
+    auto round = [&](uint32_t seed) {
+        FakeStream st;
+        for (size_t n : {size_t(1), Stager::kChunk, Stager::kChunk * Stager::kRing + 1, Stager::kLarge,
+                         Stager::kLarge + Stager::kChunk / 2 + 3}) {
+            const auto src = bytes(n, seed + uint32_t(n));
+            std::vector<uint8_t> dst(n, 0);
+            cudaError_t e = ring->copy(dst.data(), src.data(), n, &st);
+            if (e == cudaErrorNotReady) e = cudaMemcpyAsync(dst.data(), src.data(), n, cudaMemcpyHostToDevice, &st);
+            st.drain();
+            if (e != cudaSuccess || dst != src) ++wrong;
+        }
+    };
+    round(1);
+    if (fake.plain_copies) return 2;  // nobody else had the ring
+    std::vector<std::thread> ts;
+    for (uint32_t k = 0; k < 3; ++k) ts.emplace_back(round, 10 * k);
+    for (auto& t : ts) t.join();
+    return wrong ? 1 : 0;
+}
+
+int main(int argc, char** argv) {
+    const std::string mode = argc > 1 ? argv[1] : "";
+    if (mode == "data") return data();
+    return 100;
+}

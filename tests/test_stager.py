@@ -1,0 +1,25 @@
+"""The ring that large uploads go through (stager.h), compiled against a stand-in for
+the CUDA runtime: no GPU, and the stream and its errors are the test's."""
+import subprocess
+from pathlib import Path
+
+import pytest
+
+TESTS = Path(__file__).resolve().parent
+
+
+@pytest.fixture(scope="module")
+def program(tmp_path_factory):
+    out = tmp_path_factory.mktemp("stager") / "check"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", "-I", str(TESTS / "fake_cuda"),
+                    "-I", str(TESTS.parent / "tileink_b200" / "csrc"), str(TESTS / "stager_check.cpp"), "-o", str(out)],
+                   check=True)
+    return out
+
+
+def check(program, mode):
+    assert subprocess.run([str(program), mode], timeout=120).returncode == 0
+
+
+def test_uploads_arrive_whole(program):
+    check(program, "data")

@@ -14,18 +14,21 @@
 
 namespace tk {
 
-// A copy from pageable memory goes through the driver's own pinned buffer, one
-// host thread filling it: 14 GB/s measured, against 49 from pinned memory. With
-// the ring a page of 20,000 glyph outlines (77 MB of elements) takes 7.9 ms from
-// record to image, without it 10.4.
+// A copy from pageable memory goes through the driver's own pinned buffer, one host
+// thread filling it: 11 GB/s, or 20 where the source is in the CPU's caches, against 49
+// from pinned memory. With the ring a page of 20,000 glyph outlines (77 MB of elements)
+// takes 7.4 ms from record to image, without it 10.4.
+// Two threads beside the caller's fill it: with six, and chunks of 256 KB, waking them and
+// their turns at the chunks cost 0.3 ms a copy, and 16 MB from the caches took 1.09 ms,
+// through the driver 0.84; now 0.85 (24 MB 1.08 against 1.25; not cached 16 MB 1.00 against
+// 1.53, 128 MB 5.6 against 11.9). Below kLarge the driver is as fast.
 // The ring and its threads are shared by the contexts of a device: made for a
 // context whose large uploads come to kPays, given back with the last context
-// that used them. 2 MB take about 1.5 ms to make (8 MB: 6 ms), which 32 MB through
-// them win back. One copy runs at a time; a second one does not wait, and goes the
-// driver's way.
+// that used them. 4 MB take about 2.7 ms to make, which 64 MB through them win back. One
+// copy runs at a time; a second one does not wait, and goes the driver's way.
 class Stager {
   public:
-    static constexpr size_t kChunk = 256u << 10, kRing = 8, kLarge = 8u << 20, kPays = 32u << 20;
+    static constexpr size_t kChunk = 512u << 10, kRing = 8, kLarge = 16u << 20, kPays = 64u << 20;
 
     // The ring of `device` (the current one); null when another device has it or
     // it cannot be made.
@@ -106,7 +109,7 @@ class Stager {
 
     bool start() {
         const unsigned cores = std::thread::hardware_concurrency();
-        const size_t want = cores >= 16 ? 6 : (cores >= 4 ? cores / 2 : 1);
+        const size_t want = cores >= 4 ? 2 : 1;
         bool ok = cudaHostAlloc(reinterpret_cast<void**>(&ring_), kRing * kChunk, cudaHostAllocDefault) == cudaSuccess;
         if (!ok) ring_ = nullptr;
         for (size_t k = 0; ok && k < kRing; ++k)
