@@ -44,8 +44,28 @@ static int data() {
     return wrong ? 1 : 0;
 }
 
+// An upload behind a stream that is busy: the CPU time of 400 ms of waiting, in per cent of one core.
+static int busy() {
+    auto ring = Stager::of(0);
+    FakeStream st;
+    const size_t n = Stager::kChunk * Stager::kRing * 4;
+    const auto src = bytes(n, 5);
+    std::vector<uint8_t> dst(n, 0);
+    st.gate(false);
+    std::thread t([&] { ring->copy(dst.data(), src.data(), n, &st); });
+    rest(300);  // the ring is full
+    const std::clock_t c0 = std::clock();
+    rest(400);
+    const double used = double(std::clock() - c0) / CLOCKS_PER_SEC / 0.4;
+    st.gate(true);
+    t.join();
+    std::printf("%.1f%% of a core\n", 100.0 * used);
+    return dst != src ? 1 : used > 0.25 ? 2 : 0;
+}
+
 int main(int argc, char** argv) {
     const std::string mode = argc > 1 ? argv[1] : "";
     if (mode == "data") return data();
+    if (mode == "busy") return busy();
     return 100;
 }

@@ -23,3 +23,7 @@ def check(program, mode):
 
 def test_uploads_arrive_whole(program):
     check(program, "data")
+
+
+def test_fillers_sleep_while_the_stream_is_busy(program):
+    check(program, "busy")

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <chrono>
 #include <condition_variable>
 #include <cstdint>
 #include <cstring>
@@ -29,6 +30,7 @@ namespace tk {
 class Stager {
   public:
     static constexpr size_t kChunk = 512u << 10, kRing = 8, kLarge = 16u << 20, kPays = 64u << 20;
+    static constexpr std::chrono::microseconds kPatience{100};
 
     // The ring of `device` (the current one); null when another device has it or
     // it cannot be made.
@@ -89,12 +91,14 @@ class Stager {
             if (k + 1 >= kRing / 2 && k + kRing / 2 < n) {
                 const size_t back = k + 1 - kRing / 2;
                 if (e == cudaSuccess) e = cudaEventSynchronize(done_[back % kRing]);
-                limit_.store(back + 1 + kRing, std::memory_order_release);
+                limit_.store(back + 1 + kRing);
+                if (waiting_.load()) wake_fillers();
             }
         }
         {
             std::unique_lock<std::mutex> lock(m_);
             chunks_ = 0;  // a thread that wakes from now on finds nothing
+            room_.notify_all();
             idle_.wait(lock, [&] { return active_ == 0; });
         }
         // the last copy out of the ring ends after the others (one stream)
@@ -138,7 +142,7 @@ class Stager {
     bool fill_one(size_t n) {
         size_t k = next_.load(std::memory_order_relaxed);
         do {
-            if (k >= n || limit_.load(std::memory_order_acquire) <= k) return false;
+            if (k >= n || limit_.load() <= k) return false;
         } while (!next_.compare_exchange_weak(k, k + 1, std::memory_order_relaxed));
         const size_t at = k * kChunk, len = bytes_ - at < kChunk ? bytes_ - at : kChunk;
         std::memcpy(ring_ + (k % kRing) * kChunk, src_ + at, len);
@@ -146,6 +150,15 @@ class Stager {
         return true;
     }
 
+    // (limit_ is stored before waiting_ is read, and a thread counts itself in waiting_
+    // before it looks at limit_, both in one order for all: one of them sees the other)
+    void wake_fillers() {
+        { std::lock_guard<std::mutex> lock(m_); }
+        room_.notify_all();
+    }
+
+    // While the ring is full a thread yields for kPatience (the copy engine frees a slot every
+    // 10 us) and then sleeps: the stream may have a long frame to do before the copies.
     void work() {
         uint64_t seen = 0;
         std::unique_lock<std::mutex> lock(m_);
@@ -157,8 +170,21 @@ class Stager {
             if (!n) continue;  // done without this thread
             ++active_;
             lock.unlock();
-            while (next_.load(std::memory_order_relaxed) < n)
-                if (!fill_one(n)) std::this_thread::yield();
+            auto since = std::chrono::steady_clock::now();
+            while (next_.load(std::memory_order_relaxed) < n) {
+                if (fill_one(n)) {
+                    since = std::chrono::steady_clock::now();
+                } else if (std::chrono::steady_clock::now() - since < kPatience) {
+                    std::this_thread::yield();
+                } else {
+                    lock.lock();
+                    ++waiting_;
+                    room_.wait(lock, [&] { return !chunks_ || next_.load() >= n || limit_.load() > next_.load(); });
+                    --waiting_;
+                    lock.unlock();
+                    since = std::chrono::steady_clock::now();
+                }
+            }
             lock.lock();
             if (--active_ == 0) idle_.notify_one();
         }
@@ -171,9 +197,10 @@ class Stager {
     std::vector<std::thread> threads_;
     // the copy in progress
     std::mutex m_;
-    std::condition_variable wake_, idle_;
+    std::condition_variable wake_, room_, idle_;
     uint64_t job_ = 0;
     size_t active_ = 0;  // threads in it
+    std::atomic<size_t> waiting_{0};  // of them, those that sleep until a slot is free
     size_t chunks_ = 0;
     bool quit_ = false;
     const uint8_t* src_ = nullptr;
