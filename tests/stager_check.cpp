@@ -63,9 +63,46 @@ static int busy() {
     return dst != src ? 1 : used > 0.25 ? 2 : 0;
 }
 
+// A copy out of the ring that fails, behind a busy stream: the error comes back, and the
+// chunks that were issued before arrive as they were, whatever the ring does next.
+static int fail() {
+    auto ring = Stager::of(0);
+    FakeStream st;
+    const size_t n = Stager::kChunk * Stager::kRing * 4;
+    const auto src = bytes(n, 6), other = bytes(n, 7);
+    std::vector<uint8_t> dst(n, 0), dst2(n, 0);
+    for (int at : {0, 2, int(Stager::kRing) + 1}) {
+        std::fill(dst.begin(), dst.end(), uint8_t(0));
+        fake.ring_copies = 0;
+        fake.fail_copy = at;
+        // up to the half of the ring after which the copy itself waits for the stream
+        const bool closed = at < int(Stager::kRing) / 2;
+        if (closed) st.gate(false);
+        cudaError_t e = cudaSuccess;
+        std::thread t([&] { e = ring->copy(dst.data(), src.data(), n, &st); });
+        if (closed) {
+            rest(200);
+            st.gate(true);
+        }
+        t.join();
+        st.drain();
+        fake.fail_copy = -1;
+        const size_t sent = size_t(at) * Stager::kChunk;
+        if (e != cudaErrorInvalidValue) return 1;
+        if (std::memcmp(dst.data(), src.data(), sent)) return 2;
+        for (size_t i = sent; i < n; ++i)
+            if (dst[i]) return 3;
+        if (ring->copy(dst2.data(), other.data(), n, &st) != cudaSuccess) return 4;
+        st.drain();
+        if (dst2 != other) return 5;
+    }
+    return 0;
+}
+
 int main(int argc, char** argv) {
     const std::string mode = argc > 1 ? argv[1] : "";
     if (mode == "data") return data();
     if (mode == "busy") return busy();
+    if (mode == "fail") return fail();
     return 100;
 }

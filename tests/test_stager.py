@@ -27,3 +27,7 @@ def test_uploads_arrive_whole(program):
 
 def test_fillers_sleep_while_the_stream_is_busy(program):
     check(program, "busy")
+
+
+def test_a_failed_copy_leaves_the_slots_in_flight_alone(program):
+    check(program, "fail")

@@ -78,32 +78,35 @@ class Stager {
         }
         wake_.notify_all();
         cudaError_t e = cudaSuccess;
-        for (size_t k = 0; k < n; ++k) {
+        for (size_t k = 0; k < n && e == cudaSuccess; ++k) {
             // until chunk k is in its slot this thread fills chunks too
             while (filled_[k % kRing].load(std::memory_order_acquire) != k + 1)
                 if (!fill_one(n)) std::this_thread::yield();
             const size_t at = k * kChunk, len = bytes - at < kChunk ? bytes - at : kChunk, slot = k % kRing;
-            // (a failed copy leaves the rest to drain unsent)
-            if (e == cudaSuccess)
-                e = cudaMemcpyAsync(static_cast<uint8_t*>(dst) + at, ring_ + slot * kChunk, len, cudaMemcpyHostToDevice, st);
+            e = cudaMemcpyAsync(static_cast<uint8_t*>(dst) + at, ring_ + slot * kChunk, len, cudaMemcpyHostToDevice, st);
             if (e == cudaSuccess) e = cudaEventRecord(done_[slot], st);
             // the slot half a ring back is refilled once its copy is done
-            if (k + 1 >= kRing / 2 && k + kRing / 2 < n) {
+            if (e == cudaSuccess && k + 1 >= kRing / 2 && k + kRing / 2 < n) {
                 const size_t back = k + 1 - kRing / 2;
-                if (e == cudaSuccess) e = cudaEventSynchronize(done_[back % kRing]);
+                e = cudaEventSynchronize(done_[back % kRing]);
+                if (e != cudaSuccess) break;
                 limit_.store(back + 1 + kRing);
                 if (waiting_.load()) wake_fillers();
             }
         }
+        next_.store(n);  // after an error no chunk is taken any more: the slots may still be read
         {
             std::unique_lock<std::mutex> lock(m_);
             chunks_ = 0;  // a thread that wakes from now on finds nothing
             room_.notify_all();
             idle_.wait(lock, [&] { return active_ == 0; });
         }
+        if (e != cudaSuccess) {
+            cudaStreamSynchronize(st);  // the copies that were issued, out of slots that the next one fills
+            return e;
+        }
         // the last copy out of the ring ends after the others (one stream)
-        const cudaError_t last = cudaEventSynchronize(done_[(n - 1) % kRing]);
-        return e == cudaSuccess ? last : e;
+        return cudaEventSynchronize(done_[(n - 1) % kRing]);
     }
 
   private:
