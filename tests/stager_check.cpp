@@ -1,4 +1,5 @@
 // The upload ring on the CPU (tests/test_stager.py): stager_check MODE, 0 when it holds.
+#include <algorithm>
 #include <chrono>
 #include <cstdio>
 #include <ctime>
@@ -7,6 +8,9 @@
 #include "stager.h"
 
 using tk::Stager;
+using tk::Uploads;
+
+static bool no_ring = false;
 
 static std::vector<uint8_t> bytes(size_t n, uint32_t seed) {
     std::vector<uint8_t> v(n);
@@ -22,7 +26,7 @@ static void rest(int ms) { std::this_thread::sleep_for(std::chrono::milliseconds
 
 // Uploads of the sizes from several threads through one ring, as the library makes them.
 static int data() {
-    auto ring = Stager::of(0);
+    auto ring = Stager::of(0, no_ring);
     std::atomic<int> wrong{0};
     auto round = [&](uint32_t seed) {
         FakeStream st;
@@ -46,7 +50,7 @@ static int data() {
 
 // An upload behind a stream that is busy: the CPU time of 400 ms of waiting, in per cent of one core.
 static int busy() {
-    auto ring = Stager::of(0);
+    auto ring = Stager::of(0, no_ring);
     FakeStream st;
     const size_t n = Stager::kChunk * Stager::kRing * 4;
     const auto src = bytes(n, 5);
@@ -66,7 +70,7 @@ static int busy() {
 // A copy out of the ring that fails, behind a busy stream: the error comes back, and the
 // chunks that were issued before arrive as they were, whatever the ring does next.
 static int fail() {
-    auto ring = Stager::of(0);
+    auto ring = Stager::of(0, no_ring);
     FakeStream st;
     const size_t n = Stager::kChunk * Stager::kRing * 4;
     const auto src = bytes(n, 6), other = bytes(n, 7);
@@ -99,10 +103,44 @@ static int fail() {
     return 0;
 }
 
+// A context's uploads: which of them take the ring, and that a ring that cannot be made is
+// asked for once.
+static int context() {
+    FakeStream st;
+    const size_t n = Stager::kLarge, enough = Stager::kPays / n;
+    const auto src = bytes(n + 7, 8);
+    std::vector<uint8_t> dst(n + 7);
+    auto put = [&](Uploads& u, size_t len) {
+        std::fill(dst.begin(), dst.end(), uint8_t(0));
+        if (u.copy(0, dst.data(), src.data(), len, &st) != cudaSuccess) return false;
+        st.drain();
+        return std::equal(dst.begin(), dst.begin() + len, src.begin());
+    };
+    {
+        Uploads u;
+        fake.fail_alloc = true;
+        for (size_t k = 0; k < 3 * enough; ++k)
+            if (!put(u, n)) return 1;
+        if (fake.host_allocs != 1 || fake.ring_copies != 0) return 2;
+        fake.fail_alloc = false;
+    }
+    Uploads u;
+    fake.host_allocs = 0;
+    for (size_t k = 0; k + 1 < enough; ++k)
+        if (!put(u, n)) return 3;
+    if (!put(u, n - 1) || fake.host_allocs != 0) return 4;  // not large, and not yet enough
+    if (!put(u, n) || fake.host_allocs != 1 || fake.ring_copies != int(n / Stager::kChunk)) return 5;
+    if (!put(u, n + 7) || fake.ring_copies != int(2 * (n / Stager::kChunk) + 1)) return 6;
+    const int before = fake.ring_copies;
+    if (!put(u, n - 1) || fake.ring_copies != before) return 7;
+    return 0;
+}
+
 int main(int argc, char** argv) {
     const std::string mode = argc > 1 ? argv[1] : "";
     if (mode == "data") return data();
     if (mode == "busy") return busy();
     if (mode == "fail") return fail();
+    if (mode == "context") return context();
     return 100;
 }

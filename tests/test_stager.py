@@ -31,3 +31,7 @@ def test_fillers_sleep_while_the_stream_is_busy(program):
 
 def test_a_failed_copy_leaves_the_slots_in_flight_alone(program):
     check(program, "fail")
+
+
+def test_a_context_takes_the_ring_where_it_pays_and_asks_once(program):
+    check(program, "context")

@@ -239,8 +239,7 @@ struct tk_ctx {
     size_t ev_used = 0;
     std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> marks;
     FlattenScratch flat;
-    std::shared_ptr<tk::Stager> stager;  // large uploads from pageable memory
-    uint64_t large_bytes = 0;            // of such uploads so far
+    tk::Uploads uploads;
     // incremental rendering: whether `image` holds the last single-scene
     // frame (and its size and clear colour), and the redrawn tiles of the
     // frame in progress (null outside tk_render_incremental)
@@ -304,17 +303,7 @@ void upload(DBuf<T>& b, const T* src, size_t n, cudaStream_t st) {
 
 // A copy that may be large, from memory of the caller's.
 void copy_in(tk_ctx* c, void* dst, const void* src, size_t bytes, cudaStream_t st) {
-    if (!bytes) return;
-    if (tk::Stager::wants(src, bytes)) {
-        c->large_bytes += bytes;
-        if (!c->stager && c->large_bytes >= tk::Stager::kPays) c->stager = tk::Stager::of(c->device);
-        const cudaError_t e = c->stager ? c->stager->copy(dst, src, bytes, st) : cudaErrorNotReady;
-        if (e != cudaErrorNotReady) {
-            TK_CUDA(e);
-            return;
-        }
-    }
-    TK_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
+    if (bytes) TK_CUDA(c->uploads.copy(c->device, dst, src, bytes, st));
 }
 template <class T>
 void upload(tk_ctx* c, DBuf<T>& b, const T* src, size_t n, cudaStream_t st) {

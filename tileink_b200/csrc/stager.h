@@ -32,23 +32,26 @@ class Stager {
     static constexpr size_t kChunk = 512u << 10, kRing = 8, kLarge = 16u << 20, kPays = 64u << 20;
     static constexpr std::chrono::microseconds kPatience{100};
 
-    // The ring of `device` (the current one); null when another device has it or
-    // it cannot be made.
-    static std::shared_ptr<Stager> of(int device) {
+    // The ring of `device` (the current one); null when another device has it, or when it
+    // cannot be made (`failed`).
+    static std::shared_ptr<Stager> of(int device, bool& failed) {
         static std::mutex m;
         static std::weak_ptr<Stager> shared;
         std::lock_guard<std::mutex> lock(m);
         std::shared_ptr<Stager> s = shared.lock();
         if (!s) {
             s = std::shared_ptr<Stager>(new Stager(device));
-            if (!s->start()) return nullptr;
+            if (!s->start()) {
+                failed = true;
+                return nullptr;
+            }
             shared = s;
         }
         return s->device_ == device ? s : nullptr;
     }
     ~Stager() { stop(); }
 
-    // Whether src should go through the ring: large, and not pinned already.
+    // Whether src should go through a ring: large, and not pinned already.
     static bool wants(const void* src, size_t bytes) {
         if (bytes < kLarge) return false;
         cudaPointerAttributes at{};
@@ -210,6 +213,27 @@ class Stager {
     size_t bytes_ = 0;
     std::atomic<size_t> next_{0}, limit_{0};  // chunks taken; chunks whose slots are free
     std::atomic<size_t> filled_[kRing] = {};  // per slot, 1 + the chunk it holds
+};
+
+// The uploads of one context from the caller's memory.
+class Uploads {
+  public:
+    // dst[0, bytes) = src on `st`: through the device's ring (the current one's) where that
+    // pays, and as cudaMemcpyAsync does it otherwise.
+    cudaError_t copy(int device, void* dst, const void* src, size_t bytes, cudaStream_t st) {
+        if (Stager::wants(src, bytes)) {
+            large_ += bytes;
+            if (!ring_ && !failed_ && large_ >= Stager::kPays) ring_ = Stager::of(device, failed_);
+            const cudaError_t e = ring_ ? ring_->copy(dst, src, bytes, st) : cudaErrorNotReady;
+            if (e != cudaErrorNotReady) return e;
+        }
+        return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    }
+
+  private:
+    std::shared_ptr<Stager> ring_;
+    uint64_t large_ = 0;   // bytes of large uploads so far
+    bool failed_ = false;  // no ring could be made: not tried again
 };
 
 }  // namespace tk
