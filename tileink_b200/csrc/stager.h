@@ -2,6 +2,7 @@
 // of pinned chunks while the copy engine drains it.
 #pragma once
 #include <cuda_runtime.h>
+#include <pthread.h>
 
 #include <atomic>
 #include <chrono>
@@ -166,6 +167,7 @@ class Stager {
     // While the ring is full a thread yields for kPatience (the copy engine frees a slot every
     // 10 us) and then sleeps: the stream may have a long frame to do before the copies.
     void work() {
+        pthread_setname_np(pthread_self(), "tileink-upload");
         uint64_t seen = 0;
         std::unique_lock<std::mutex> lock(m_);
         for (;;) {
