@@ -208,8 +208,7 @@ struct tk_ctx {
     DBuf<uint32_t> counts, cursors, bumps, misc;
     DBuf<tk_segment_range> ranges;
     DBuf<tk::SegmentRec> segments;
-    DBuf<tk::PaintInfo> paints;  // per draw, built at upload
-    DBuf<tk::DrawInfo> infos;    // per draw, built at upload
+    DBuf<tk::PaintInfo> paints;  // per draw, built at upload; the DrawInfo of every draw behind them
     uint64_t segment_needed = 0;  // device plan: total from the last frame
     DBuf<uint32_t> image, temp, low;  // target, blur temporary, reduced-resolution blur surface
     tk::ProgressiveScratch prog_scratch;  // progressive blur levels (grown on demand)
@@ -632,6 +631,8 @@ void validate_and_plan(tk_ctx* c, const tk_scene_desc& d) {
     c->tile_draw_refs = refs;
 }
 
+tk::DrawInfo* draw_infos(tk_ctx* c) { return reinterpret_cast<tk::DrawInfo*>(c->paints.ptr + c->draw_count); }
+
 tk::SceneView view(tk_ctx* c) {
     tk::SceneView s{};
     s.lines = c->lines.ptr;
@@ -673,7 +674,7 @@ tk::SceneView view(tk_ctx* c) {
     s.error = c->misc.ptr;
     s.seg_line = c->want_seg_line ? c->seg_line.ptr : nullptr;
     s.paints = c->paints.ptr;
-    s.infos = c->infos.ptr;
+    s.infos = draw_infos(c);
     s.emit_order = c->emit_order.ptr;
     s.emit_ticket = c->misc.ptr + 4;
     s.longest_path = c->longest_path;
@@ -724,6 +725,13 @@ uint32_t read_word(tk_ctx* c, const uint32_t* dptr) {
 }
 
 // Paths by decreasing line count (stable), for scan_emit's path queue.
+// The per-draw tables of the uploaded records.
+void make_draw_tables(tk_ctx* c, const uint4* images, uint32_t image_count) {
+    constexpr size_t kInfos = sizeof(tk::PaintInfo) / sizeof(tk::DrawInfo);
+    c->paints.reserve(c->draw_count + (c->draw_count + kInfos - 1) / kInfos);
+    tk::launch_draw_tables(view(c), images, image_count, c->paints.ptr, draw_infos(c), c->stream);
+}
+
 void upload_emit_order(tk_ctx* c) {
     // Paths longest first, ties in path order: a stable sort by descending
     // line count, done as an LSD radix sort of the inverted counts (16 bits a
@@ -847,13 +855,9 @@ void do_upload(tk_ctx* c, const tk_scene_desc& scene, const tk_flatten_desc* fl 
     }
     if (!fl) side_copies();
     TK_CUDA(cudaStreamWaitEvent(st, c->ev_copy, 0));
-    c->paints.reserve(d.draw_count);
-    tk::launch_paint_table(c->draws.ptr, d.draw_count, c->brush.ptr, d.brush_word_count,
-                           uint32_t(c->sdf_shadow_base), c->image_tab.ptr, d.image_count, c->paints.ptr, st);
-    upload(c->layers, d.layers, d.layer_count, st);
     upload(c->batch_ids, d.draw_batch_ids, d.draw_count, st);
-    c->infos.reserve(d.draw_count);
-    tk::launch_draw_table(view(c), st);
+    make_draw_tables(c, c->image_tab.ptr, d.image_count);
+    upload(c->layers, d.layers, d.layer_count, st);
     upload(c->order, d.draw_order, d.draw_order_count, st);
     upload(c->items, c->h_items.data(), c->h_items.size(), st);
     upload_emit_order(c);
@@ -1549,13 +1553,9 @@ void do_batch_upload(tk_ctx* c, const tk_scene_desc* scenes, uint32_t n) {
     upload(c->draws, draws.data(), draws.size(), st);
     upload(c->brush, brush.data(), brush.size(), st);
     upload(c->sdf, sdf.data(), sdf.size(), st);
-    c->paints.reserve(draws.size());
-    tk::launch_paint_table(c->draws.ptr, uint32_t(draws.size()), c->brush.ptr, brush.size(),
-                           uint32_t(c->sdf_shadow_base), nullptr, 0u, c->paints.ptr, st);
-    upload(c->layers, layers.data(), layers.size(), st);
     upload(c->batch_ids, batch_ids.data(), batch_ids.size(), st);
-    c->infos.reserve(draws.size());
-    tk::launch_draw_table(view(c), st);
+    make_draw_tables(c, nullptr, 0u);
+    upload(c->layers, layers.data(), layers.size(), st);
     upload(c->order, order.data(), order.size(), st);
     rebuild_items(c);
     upload_emit_order(c);
@@ -1687,7 +1687,6 @@ void tk_ctx_destroy(tk_ctx* c) {
     c->d_scenes.release(); c->bin_scene.release(); c->tile_scene.release();
     c->flat.release();
     c->paints.release();
-    c->infos.release();
     c->tile_active.release();
     c->tile_list.release();
     DiffState& D = c->diff;

@@ -13,7 +13,7 @@
 // in the tile contributes TK_PTCL_BATCH_BEGIN{segment_start = batch id,
 // segment_end = record count, color = kind | skip << 3} followed by the
 // reference batch stream without its END; one END closes the tile.
-// What the walk needs of a draw is decoded once per upload (k_draw_table).
+// What the walk needs of a draw is decoded once per upload (draws.cuh).
 //
 // What bounds it is latency: a candidate's range and backdrop are one load deep,
 // and a lane per candidate keeps 32 of them in flight per tile. One thread per
@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 
 #include "device.cuh"
+#include "draws.cuh"
 #include "kernels.h"
 #include "sdf.cuh"
 
@@ -38,17 +39,6 @@ constexpr int kQuadThreads = kQuadSide * kQuadSide;
 constexpr uint32_t kPrefetchCount = 8, kPrefetchEmit = 4;  // a tile's loads in flight, counting and emitting
 constexpr uint32_t kCandidates = 256;  // staged at a time, one per thread (their numbers are bytes)
 constexpr uint32_t kChunkClassColor = 1u, kChunkClassSdf = 2u, kChunkClassOther = 4u, kChunkClassOccluder = 8u;
-// DrawInfo::meta bits (staged candidates: the batch ordinal in the pass above them, from bit kMetaBatchShift)
-constexpr uint32_t kMetaPath = 16u, kMetaSolid = 32u, kMetaSdf = 64u, kMetaSdfSolidClass = 128u, kMetaGlyph = 256u;
-constexpr uint32_t kMetaBatchShift = 9u;
-// DrawInfo::py bits of an SDF draw (px holds its first SDF word)
-constexpr uint32_t kSdfPlain = 256u, kSdfIdentity = 512u, kSdfImage = 1024u;
-__device__ __forceinline__ uint32_t tile_min_(int32_t px, uint32_t lim) {
-    return px > 0 ? min(uint32_t(px) / TK_TILE_SIZE, lim) : 0u;
-}
-__device__ __forceinline__ uint32_t tile_max_(int32_t px, uint32_t lim) {
-    return px > 0 ? min((uint32_t(px) + TK_TILE_SIZE - 1u) / TK_TILE_SIZE, lim) : 0u;
-}
 
 // ---------------------------------------------------------------------------
 // Binning.
@@ -310,71 +300,6 @@ static __device__ __noinline__ uint32_t sdf_particle(const tk_draw_record* draws
     // full_tile_solid, then full_tile_image (coarse/paint.hlsli:27-34)
     if (!sdf_rect_covers(sdf + word, ex, ey, tx, ty)) return TK_PTCL_SDF;
     return (meta & kMetaSolid) ? TK_PTCL_COLOR : TK_PTCL_IMAGE;
-}
-
-// What binning and the candidate walk need of draw `di` (struct DrawInfo).
-__global__ void k_draw_table(Ctx c, uint32_t draw_count, const uint32_t* __restrict__ batch_ids, DrawInfo* out) {
-    const uint32_t di = blockIdx.x * blockDim.x + threadIdx.x;
-    if (di >= draw_count) return;
-    const tk_draw_record& d = c.draws[di];
-    DrawInfo info{};
-    info.batch = batch_ids[di];
-    info.tx = tile_min_(d.pixel_bounds.x0, 65535u) | (tile_max_(d.pixel_bounds.x1, 65535u) << 16);
-    info.ty = tile_min_(d.pixel_bounds.y0, 65535u) | (tile_max_(d.pixel_bounds.y1, 65535u) << 16);
-    bool valid_path = d.path_id != TK_INVALID_INDEX && d.tag <= TK_DRAW_PATH_GLYPH && d.path_id < c.path_count;
-    if (valid_path) {
-        const tk_path_record& p = c.paths[d.path_id];
-        info.px = p.tile_x0 | (p.tile_x1 << 16);
-        info.py = p.tile_y0 | (p.tile_y1 << 16);
-        info.data_offset = p.data_offset;
-    }
-    bool color_candidate = false;
-    info.color = di;
-    // nontransparent_solid (coarse/paint.hlsli:13-17)
-    const bool solid = d.brush_offset != TK_INVALID_INDEX && brush_word(c, d.brush_offset) == TK_BRUSH_SOLID &&
-                       brush_word(c, d.brush_offset + TK_BRUSH_COLOR_WORD) != 0u;
-    // a glyph run draw gives a PTCL_GLYPH particle or none
-    // (coarse/emit_draw.hlsli:15-22)
-    const bool glyph = c.glyph_runs && d.glyph_run_id != TK_INVALID_INDEX;
-    const bool has_sdf = !glyph && (d.sdf_offset != TK_INVALID_INDEX || d.sdf_shadow_offset != TK_INVALID_INDEX);
-    uint32_t bits = 0u;
-    if (glyph) {
-        valid_path = false;
-        if (d.tag == TK_DRAW_BRUSH && d.glyph_run_id < c.glyph_run_count) {
-            const tk_glyph_run run = c.glyph_runs[d.glyph_run_id];
-            info.px = run.first;
-            info.py = run.count;
-            bits |= kMetaGlyph;
-        }
-    } else if (has_sdf) {
-        // draw_has_sdf (shared/draw.hlsli:31): only brush draws give a particle
-        valid_path = false;
-        const bool plain = d.sdf_offset != TK_INVALID_INDEX;
-        info.px = plain ? d.sdf_offset : uint32_t(c.sdf_shadow_base) + d.sdf_shadow_offset;
-        const uint32_t kind = __ldg(c.sdf + info.px);
-        const bool ident = d.transform.a == 1.0f && d.transform.b == 0.0f && d.transform.c == 0.0f &&
-                           d.transform.d == 1.0f;
-        // full_tile_image's brush test: an image pattern at full opacity
-        const bool image = d.brush_offset != TK_INVALID_INDEX &&
-                           brush_word(c, d.brush_offset) == TK_BRUSH_PATTERN_RESOURCE &&
-                           brush_word(c, d.brush_offset + TK_BRUSH_IMAGE_ALPHA_WORD) == 255u;
-        info.py = (kind & 255u) | (plain ? kSdfPlain : 0u) | (ident ? kSdfIdentity : 0u) | (image ? kSdfImage : 0u);
-        if (d.tag == TK_DRAW_BRUSH) bits |= kMetaSdf;
-        if (solid) {
-            color_candidate = true;
-            info.color = brush_word(c, d.brush_offset + TK_BRUSH_COLOR_WORD);
-        }
-        // solid_supported_sdf (coarse/paint.hlsli:21-25)
-        if (solid && plain && (kind == TK_SDF_RECT || kind == TK_SDF_CANDLESTICK || kind == TK_SDF_CHECKERBOARD))
-            bits |= kMetaSdfSolidClass;
-    } else if (d.tag == TK_DRAW_BRUSH && d.solid_rect != 0u && d.transform.b == 0.0f && d.transform.c == 0.0f && solid) {
-        color_candidate = true;
-        info.color = brush_word(c, d.brush_offset + TK_BRUSH_COLOR_WORD);
-    }
-    if (d.tag == TK_DRAW_CLIP) info.color = 0u;
-    const uint32_t rule = has_sdf ? 0u : (d.fill_rule & 1u);  // SDF particles carry rule 0
-    info.meta = (d.tag & 7u) | (rule << 3) | (valid_path ? kMetaPath : 0u) | (color_candidate ? kMetaSolid : 0u) | bits;
-    out[di] = info;
 }
 
 // A tile's stream between candidate steps. `wrappers` is TK_INVALID_INDEX for a
@@ -1002,11 +927,6 @@ Ctx coarse_ctx(const SceneView& s) {
 }
 
 }  // namespace
-
-void launch_draw_table(const SceneView& s, cudaStream_t st) {
-    if (s.draw_count)
-        k_draw_table<<<(s.draw_count + 127) / 128, 128, 0, st>>>(coarse_ctx(s), s.draw_count, s.batch_ids, s.infos);
-}
 
 // A thread per tile from this many tiles of one canvas on (4096x4096 / 50,000
 // paths, 65,536 tiles: count 4.7, emit 5.8 ms against 4.9 and 8.3 with a warp

@@ -25,6 +25,7 @@
 #include <cuda_runtime.h>
 
 #include "device.cuh"
+#include "draws.cuh"
 #include "fine.cuh"
 #include "kernels.h"
 #include "sdf.cuh"
@@ -170,25 +171,25 @@ __device__ void decode_gradient(float* g, uint4& gk, const Paint& P, uint32_t db
 }
 
 // One thread per draw: the draw's PaintInfo (solid colour, or the decoded
-// gradient of its brush under its inverse transform).
-__global__ void k_paint_table(const tk_draw_record* __restrict__ draws, uint32_t n, const uint32_t* __restrict__ brush,
-                              uint64_t brush_words, uint32_t sdf_shadow_base, const uint4* __restrict__ images,
-                              uint32_t image_count, PaintInfo* out) {
+// gradient of its brush under its inverse transform) and its DrawInfo. Both in one
+// launch: with one each an upload of a small scene took 5 us more.
+__global__ void k_draw_tables(const DrawTables t) {
     const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
-    if (d >= n) return;
-    const Paint P{brush, brush_words};
-    const uint32_t bo = draws[d].brush_offset;
+    if (d >= t.n) return;
+    const Paint P{t.brush, t.brush_words};
+    const uint32_t bo = t.draws[d].brush_offset;
     PaintInfo info{};
     // sdf_coverage_from_draw (fine/draw.hlsli:21-26): the SDF record, else the shadow record
-    const uint32_t so = draws[d].sdf_offset, ho = draws[d].sdf_shadow_offset;
-    info.sdf = so != TK_INVALID_INDEX ? so : (ho != TK_INVALID_INDEX ? sdf_shadow_base + ho : TK_INVALID_INDEX);
+    const uint32_t so = t.draws[d].sdf_offset, ho = t.draws[d].sdf_shadow_offset;
+    info.sdf = so != TK_INVALID_INDEX ? so : (ho != TK_INVALID_INDEX ? t.sdf_shadow_base + ho : TK_INVALID_INDEX);
     if (P.word(bo) == TK_BRUSH_SOLID) {
         info.paint = P.word(bo + TK_BRUSH_COLOR_WORD);
     } else {
         info.paint = kGradient;
-        decode_gradient(info.g, info.gk, P, bo, &draws[d].inverse_transform.a, images, image_count);
+        decode_gradient(info.g, info.gk, P, bo, &t.draws[d].inverse_transform.a, t.images, t.image_count);
     }
-    out[d] = info;
+    t.paints[d] = info;
+    t.infos[d] = draw_info(t, P, d);
 }
 
 // segment_row_parts (shared/coverage.hlsli:7-24) of staged segment j for
@@ -768,12 +769,13 @@ __global__ void k_star_table() {
 
 }  // namespace
 
-void launch_paint_table(const tk_draw_record* draws, uint32_t draw_count, const uint32_t* brush,
-                        uint64_t brush_words, uint32_t sdf_shadow_base, const uint4* images, uint32_t image_count,
-                        PaintInfo* out, cudaStream_t st) {
-    if (draw_count)
-        k_paint_table<<<(draw_count + 255) / 256, 256, 0, st>>>(draws, draw_count, brush, brush_words,
-                                                                sdf_shadow_base, images, image_count, out);
+void launch_draw_tables(const SceneView& s, const uint4* images, uint32_t image_count, PaintInfo* paints,
+                        DrawInfo* infos, cudaStream_t st) {
+    if (s.draw_count)
+        k_draw_tables<<<(s.draw_count + 127) / 128, 128, 0, st>>>(
+            DrawTables{s.draws, s.draw_count, s.paths, s.path_count, s.brush, s.brush_words, s.sdf,
+                       uint32_t(s.sdf_shadow_base), s.glyph_runs, s.glyph_run_count, s.batch_ids, images, image_count,
+                       paints, infos});
 }
 
 void launch_fine(const SceneView& s, const PassView& p, uint32_t* target, cudaStream_t st) {

@@ -60,7 +60,7 @@ struct alignas(16) PaintInfo {
 static_assert(sizeof(PaintInfo) == 128, "two 64-byte halves");
 
 // A draw as binning and coarse need it, decoded once per upload from the draw,
-// its path record and its brush (coarse.cu, k_draw_table).
+// its path record and its brush (draws.cuh).
 struct alignas(16) DrawInfo {
     uint32_t tx, ty;         // draw tile bbox (not clamped to the canvas): x0 | x1 << 16, y0 | y1 << 16 (read as a pair)
     uint32_t px, py;         // path tile bbox packed the same way; SDF draws: first SDF word, kind | flags;
@@ -109,8 +109,8 @@ struct SceneView {
     uint64_t segment_capacity;
     uint32_t* error;
     uint32_t* seg_line;  // optional: line index of every emitted segment
-    const PaintInfo* paints;     // per draw (launch_paint_table)
-    DrawInfo* infos;             // per draw (launch_draw_table)
+    const PaintInfo* paints;     // per draw (launch_draw_tables)
+    const DrawInfo* infos;       // per draw
     const uint32_t* emit_order;  // paths by decreasing line count (optional)
     uint32_t* emit_ticket;       // path queue of scan_emit
     uint32_t longest_path;       // the most lines of one path
@@ -211,16 +211,11 @@ void launch_fine(const SceneView& s, const PassView& p, uint32_t* target, cudaSt
 // launch_fine's kernel for scenes without SDF records and text (fine_paths.cu),
 // over `tiles` tiles (of the pass's list when it has one).
 void launch_fine_paths(const SceneView& s, const PassView& p, uint32_t* target, uint32_t tiles, cudaStream_t st);
-// The per-draw PaintInfo table of the uploaded draws and brush blob; shadow
-// records start at word sdf_shadow_base of the device SDF buffer.
+// The per-draw PaintInfo and DrawInfo tables of the uploaded scene (draws, paths, brushes,
+// SDF records with the shadow records behind them, glyph runs and batch ids).
 // images: per image of the texture table its first texel, width and height.
-void launch_paint_table(const tk_draw_record* draws, uint32_t draw_count, const uint32_t* brush,
-                        uint64_t brush_words, uint32_t sdf_shadow_base, const uint4* images, uint32_t image_count,
-                        PaintInfo* out, cudaStream_t st);
-
-// The per-draw DrawInfo table of the uploaded scene (draws, paths, brushes, SDF
-// records, glyph runs and batch ids).
-void launch_draw_table(const SceneView& s, cudaStream_t st);
+void launch_draw_tables(const SceneView& s, const uint4* images, uint32_t image_count, PaintInfo* paints,
+                        DrawInfo* infos, cudaStream_t st);
 
 // Images.
 void launch_fill(uint32_t* image, uint64_t n, uint32_t value, cudaStream_t st);
