@@ -139,8 +139,7 @@ def max_over_ranks(value: float, world: int, device: str = "cuda") -> float:
 
 
 def fp32_peak_tflops() -> float:
-    """The FP32 FMA peak measured on a B200 by fp32_probe.cu, committed in
-    profiles/fp32_peak_fma.txt."""
+    """The FP32 FMA peak measured on a B200, committed in profiles/fp32_peak_fma.txt."""
     for line in (ROOT / "profiles" / "fp32_peak_fma.txt").read_text().splitlines():
         if line.startswith("fp32_tflops "):
             return float(line.split()[1])
@@ -969,7 +968,7 @@ def main():
     dominant = max(rooflines, key=lambda k: rooflines[k]["ms"])
     roof = dict(rooflines[dominant])
     roof["kernel"] = dominant
-    roof["peak_source"] = ("measured FMA probe (fp32_probe.cu, profiles/fp32_peak_fma.txt)" if roof["bound"] == "fp32"
+    roof["peak_source"] = ("measured FMA probe (profiles/fp32_peak_fma.txt)" if roof["bound"] == "fp32"
                            else "measured (MEASURED_PEAKS.json hbm_gbs)")
     # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) from
     # the committed ncu launch list of the default 4096^2 / 50k workload; other

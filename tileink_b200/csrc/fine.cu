@@ -8,7 +8,7 @@
 // stages into shared memory, with coalesced loads and no dependent global
 // round trips per record:
 //   - the records and each fill's paint, one load of the draw's PaintInfo
-//     (decoded once per upload by k_paint_table);
+//     (decoded once per upload by k_draw_tables);
 //   - the chunk's segments and, per tile row, the compacted list of segments
 //     that cross the row (dy != 0) with their terms of segment_row_parts
 //     (shared/coverage.hlsli:7-24). A segment crosses 4-5 of the 16 rows on
@@ -784,7 +784,7 @@ void launch_fine(const SceneView& s, const PassView& p, uint32_t* target, cudaSt
     // Path-only scenes take the kernel with several pixels per thread. The
     // others stay here: a pixel's SDF shape or glyphs cost far more than the
     // record's dispatch, which is all that is shared between a thread's pixels
-    // (4096^2, 50,000 paths: 207 -> 128 ms; 2048^2, 12,500 shapes: 1.62 here,
+    // (4096^2, 50,000 paths: 207 -> 122 ms; 2048^2, 12,500 shapes: 1.62 here,
     // 1.65 there; 1280x800 glyph runs: 0.32 here, 0.49 ms there).
     if (!s.text && !s.sdf_words) return launch_fine_paths(s, p, target, T, st);
     if (s.sdf_ext) k_star_table<<<1, 32, 0, st>>>();

@@ -2,26 +2,28 @@
 // two horizontally adjacent pixels per thread (fine/main.hlsl:23-40,
 // fine/interpreter.hlsli:21-219, fine/specialized.hlsli:19-45).
 //
-// What bounds it is instruction issue: HBM is idle and a tile's records are a
-// serial chain. A record's dispatch and staging are the same for the two
+// What bounds it is its instructions: HBM is idle, and a tile's records are a
+// serial chain that uses two thirds of the issue slots; for the rest the warps wait
+// for fixed latencies and at the barriers between staging and compositing. A
+// record's dispatch and staging are the same for the two
 // pixels of a thread, the pixel arithmetic runs on f32 pairs (f32x2), and
 // coverage is evaluated by half rows of fills instead of pixel by pixel.
-// Against one pixel per thread with coverage in the record loop: 4.7 G against
-// 8.5 G warp instructions on the 2048x2048 / 6,000-path frame, 6.1 against
-// 10.1 ms; 4096x4096 / 50,000 paths 128 against 207 ms, 1283x717 / 2,500 paths
-// 1.12 against 1.99 ms, 640x360 / 240 fills 0.26 against 0.29 ms.
+// Against one pixel per thread with coverage in the record loop: 4.5 G against
+// 8.5 G warp instructions on the 2048x2048 / 6,000-path frame, 5.8 against
+// 10.1 ms; 4096x4096 / 50,000 paths 122 against 207 ms, 1283x717 / 2,500 paths
+// 1.03 against 1.99 ms, 640x360 / 240 fills 0.24 against 0.29 ms.
 // Four pixels per thread (64-thread CTAs) took 6.8 ms on the 2048 frame and
 // eight (one warp a tile) 11.1: too few warps are in flight, and half-size
 // chunks repeat the staging. The loops of the staging are not unrolled and the
-// rare records are out of line: with both inline 2 of 8.9 warps per issue waited
-// for instructions, 0.35 of 7.3 after.
+// rare records are out of line (opacity groups: in an instance of their own): with
+// both inline 2 of 8.9 warps per issue waited for instructions, 0.44 of 10.2 now.
 //
 // The tile's merged PTCL stream is processed in chunks of up to 32 records
 // whose fills together reference at most kSegs tile segments (and at most
 // kItems crossings and kBlocks blocks of products, below). Per chunk the CTA
 // stages into shared memory:
 //   - the records and each fill's solid paint (its draw's PaintInfo, decoded
-//     once per upload by k_paint_table);
+//     once per upload by k_draw_tables);
 //   - the chunk's segments, and for every (segment, row) crossing (dy != 0) an
 //     entry with its terms of segment_row_parts (shared/coverage.hlsli:7-24),
 //     listed per tile row in segment order;

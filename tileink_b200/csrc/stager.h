@@ -19,7 +19,7 @@ namespace tk {
 // A copy from pageable memory goes through the driver's own pinned buffer, one host
 // thread filling it: 11 GB/s, or 20 where the source is in the CPU's caches, against 49
 // from pinned memory. With the ring a page of 20,000 glyph outlines (77 MB of elements)
-// takes 7.4 ms from record to image, without it 10.4.
+// takes 7.0 ms from record to image, without it 10.5.
 // Two threads beside the caller's fill it: with six, and chunks of 256 KB, waking them and
 // their turns at the chunks cost 0.3 ms a copy, and 16 MB from the caches took 1.09 ms,
 // through the driver 0.84; now 0.85 (24 MB 1.08 against 1.25; not cached 16 MB 1.00 against
