@@ -133,6 +133,12 @@ static int context() {
     if (!put(u, n + 7) || fake.ring_copies != int(2 * (n / Stager::kChunk) + 1)) return 6;
     const int before = fake.ring_copies;
     if (!put(u, n - 1) || fake.ring_copies != before) return 7;
+    // arrays that several threads have just written, from kWritten on
+    for (size_t len : {Stager::kWritten - 1, Stager::kWritten}) {
+        if (u.copy(0, dst.data(), src.data(), len, &st, true) != cudaSuccess) return 8;
+        st.drain();
+        if (fake.ring_copies != before + int(len / Stager::kWritten * (Stager::kWritten / Stager::kChunk))) return 9;
+    }
     return 0;
 }
 

@@ -300,14 +300,14 @@ void upload(DBuf<T>& b, const T* src, size_t n, cudaStream_t st) {
     if (n) TK_CUDA(cudaMemcpyAsync(b.ptr, src, n * sizeof(T), cudaMemcpyHostToDevice, st));
 }
 
-// A copy that may be large, from memory of the caller's.
-void copy_in(tk_ctx* c, void* dst, const void* src, size_t bytes, cudaStream_t st) {
-    if (bytes) TK_CUDA(c->uploads.copy(c->device, dst, src, bytes, st));
+// A copy that may be large, from pageable memory (`written`: see Uploads).
+void copy_in(tk_ctx* c, void* dst, const void* src, size_t bytes, cudaStream_t st, bool written = false) {
+    if (bytes) TK_CUDA(c->uploads.copy(c->device, dst, src, bytes, st, written));
 }
 template <class T>
-void upload(tk_ctx* c, DBuf<T>& b, const T* src, size_t n, cudaStream_t st) {
+void upload(tk_ctx* c, DBuf<T>& b, const T* src, size_t n, cudaStream_t st, bool written = false) {
     b.reserve(n);
-    copy_in(c, b.ptr, src, n * sizeof(T), st);
+    copy_in(c, b.ptr, src, n * sizeof(T), st, written);
 }
 
 // Host validation of a scene against the contracts the kernels rely on.
@@ -2340,9 +2340,9 @@ int32_t tk_diff_forward(tk_ctx* c, const tk_diff_scene* sc, const float* target,
         check_error_word(c);
         const uint64_t n = uint64_t(sc->width) * sc->height;
         upload(D.colp, colp.data(), colp.size(), st);
+        upload(c, D.ep_point, ep_point.data(), ep_point.size(), st, true);
+        upload(c, D.ep_w, ep_w.data(), ep_w.size(), st, true);
         upload(c, D.target, reinterpret_cast<const float4*>(target), n, st);
-        upload(c, D.ep_point, ep_point.data(), ep_point.size(), st);
-        upload(c, D.ep_w, ep_w.data(), ep_w.size(), st);
         D.layer.reserve(n);
         D.gI.reserve(n);
         D.sums.reserve(2);

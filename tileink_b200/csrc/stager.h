@@ -23,14 +23,17 @@ namespace tk {
 // Two threads beside the caller's fill it: with six, and chunks of 256 KB, waking them and
 // their turns at the chunks cost 0.3 ms a copy, and 16 MB from the caches took 1.09 ms,
 // through the driver 0.84; now 0.85 (24 MB 1.08 against 1.25; not cached 16 MB 1.00 against
-// 1.53, 128 MB 5.6 against 11.9). Below kLarge the driver is as fast.
+// 1.53, 128 MB 5.6 against 11.9). Below kLarge the driver is as fast, except on arrays that
+// several threads have just written: they lie in those cores' caches, from which one thread
+// reads 5.5 GB/s (the 5.6 MB of weights of a differentiable step: 1.0 ms; from kWritten
+// on they take the ring, 6.2 -> 5.9 ms a step's forward).
 // The ring and its threads are shared by the contexts of a device: made for a
 // context whose large uploads come to kPays, given back with the last context
 // that used them. 4 MB take about 2.7 ms to make, which 64 MB through them win back. One
 // copy runs at a time; a second one does not wait, and goes the driver's way.
 class Stager {
   public:
-    static constexpr size_t kChunk = 512u << 10, kRing = 8, kLarge = 16u << 20, kPays = 64u << 20;
+    static constexpr size_t kChunk = 512u << 10, kRing = 8, kLarge = 16u << 20, kWritten = 4u << 20, kPays = 64u << 20;
     static constexpr std::chrono::microseconds kPatience{100};
 
     // The ring of `device` (the current one); null when another device has it, or when it
@@ -52,9 +55,9 @@ class Stager {
     }
     ~Stager() { stop(); }
 
-    // Whether src should go through a ring: large, and not pinned already.
-    static bool wants(const void* src, size_t bytes) {
-        if (bytes < kLarge) return false;
+    // Whether src should go through a ring: `least` bytes or more, and not pinned already.
+    static bool wants(const void* src, size_t bytes, size_t least) {
+        if (bytes < least) return false;
         cudaPointerAttributes at{};
         if (cudaPointerGetAttributes(&at, src) != cudaSuccess) {
             cudaGetLastError();
@@ -221,9 +224,9 @@ class Stager {
 class Uploads {
   public:
     // dst[0, bytes) = src on `st`: through the device's ring (the current one's) where that
-    // pays, and as cudaMemcpyAsync does it otherwise.
-    cudaError_t copy(int device, void* dst, const void* src, size_t bytes, cudaStream_t st) {
-        if (Stager::wants(src, bytes)) {
+    // pays, and as cudaMemcpyAsync does it otherwise. written: by several threads, just now.
+    cudaError_t copy(int device, void* dst, const void* src, size_t bytes, cudaStream_t st, bool written = false) {
+        if (Stager::wants(src, bytes, written ? Stager::kWritten : Stager::kLarge)) {
             large_ += bytes;
             if (!ring_ && !failed_ && large_ >= Stager::kPays) ring_ = Stager::of(device, failed_);
             const cudaError_t e = ring_ ? ring_->copy(dst, src, bytes, st) : cudaErrorNotReady;
